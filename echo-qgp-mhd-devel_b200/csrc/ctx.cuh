@@ -56,14 +56,11 @@ struct EchoCtx {
   // [1 - on] = vold / uold
   int keep_old, kold, on;
   double *d_oldv[2], *d_oldu[2];
-  // product build: how the face sweeps run: 0 one thread per face, 8 or 16
-  // the cell-centred kernel in segments of that many cells
+  // cells along the sweep of a y or eta tile: 0 the library's choice, 8 or 16
+  // (echo_gpu_set_faces)
   int face_mode;
-  // concurrent sweeps: the y and eta sweeps of a stage run on two side
-  // streams forked from and joined back into `stream` (par_sweeps = 1)
+  // one launch for all the sweeps of a stage (1), or one each in order
   int par_sweeps;
-  cudaStream_t side[2];
-  cudaEvent_t ev_fork, ev_join[2];
   // echo_gpu_advance_host: the host copy of u runs on copy_stream and ev_u
   // marks its end; while wait_u is set, the next step's first u access
   // waits for it (join_u)
@@ -104,7 +101,7 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
 namespace echo {
 
 template <int KIND>
-void launch_faces(EchoCtx* c, int dir);
+void launch_faces(EchoCtx* c, int mask);
 template <int KIND>
 void launch_update(EchoCtx* c, int irk, int mode, double* du_out);
 // what: 1 = repair only, 2 = smoothing only, 3 = both

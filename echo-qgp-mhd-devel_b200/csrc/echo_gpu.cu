@@ -152,7 +152,7 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
   return ECHO_OK;
 }
 
-// whether the sweeps of a stage run concurrently (launch_sweeps)
+// whether the sweeps of a stage are one launch (launch_sweeps)
 #ifndef ECHO_PAR_SWEEPS
 #define ECHO_PAR_SWEEPS 1
 #endif
@@ -187,37 +187,22 @@ static void launch_scalars(EchoCtx* c, int irk, int mode = 0) {
   stage_scalars_kernel<<<1, 1, 0, c->stream>>>(S);
 }
 
-// The flux sweeps of a stage.  They are independent of each other: each
-// reads v and writes its own face fluxes and its own signal-speed slots
-// (amax_bits[d], aflux[d]).  With par_sweeps the first runs on `stream` and
-// the others on the side streams, forked from and joined back into it, so
-// that the partial last wave of one overlaps the others (under stream
-// capture the fork and join become branches of the step graph).  Per-kernel
-// profiling keeps them in order, so that each can be timed.
+// The flux sweeps of a stage: one launch for all directions, or, with
+// par_sweeps off and for per-kernel profiling, one for each in order.
 static void launch_sweeps(EchoCtx* c) {
-  int dirs[3], nd = 0;
-  for (int d = 0; d < 3; d++) {
-    int n = d == 0 ? c->g.nx : d == 1 ? c->g.ny : c->g.nz;
-    if (n > 1) dirs[nd++] = d;
-  }
-  if (!c->par_sweeps || c->marks || nd < 2) {
-    for (int j = 0; j < nd; j++) {
-      DISPATCH(c, launch_faces, c, dirs[j]);
-      mark(c, PK_FACES_X + dirs[j]);
-    }
+  int mask = 0;
+  for (int d = 0; d < 3; d++)
+    if ((d == 0 ? c->g.nx : d == 1 ? c->g.ny : c->g.nz) > 1) mask |= 1 << d;
+  if (!mask) return;
+  if (c->par_sweeps && !c->marks) {
+    DISPATCH(c, launch_faces, c, mask);
     return;
   }
-  cudaEventRecord(c->ev_fork, c->stream);
-  const cudaStream_t main = c->stream;
-  for (int j = 1; j < nd; j++) {
-    cudaStreamWaitEvent(c->side[j - 1], c->ev_fork, 0);
-    c->stream = c->side[j - 1];
-    DISPATCH(c, launch_faces, c, dirs[j]);
-    cudaEventRecord(c->ev_join[j - 1], c->stream);
-  }
-  c->stream = main;
-  DISPATCH(c, launch_faces, c, dirs[0]);
-  for (int j = 1; j < nd; j++) cudaStreamWaitEvent(c->stream, c->ev_join[j - 1], 0);
+  for (int d = 0; d < 3; d++)
+    if (mask >> d & 1) {
+      DISPATCH(c, launch_faces, c, 1 << d);
+      mark(c, PK_FACES_X + d);
+    }
 }
 
 // the flux sweeps of a stage; the CFL maxima start from zero
@@ -405,11 +390,6 @@ int echo_gpu_init(const EchoParams* p, const double* eos_table, int n_eos, EchoC
   c->nfaces[2] = (size_t)p->nx * p->ny * (p->nz + 1);
   size_t nvc = (size_t)c->nv * c->g.ncell;
   CK(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  CK(cudaStreamCreateWithFlags(&c->side[0], cudaStreamNonBlocking));
-  CK(cudaStreamCreateWithFlags(&c->side[1], cudaStreamNonBlocking));
-  CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&c->ev_join[0], cudaEventDisableTiming));
-  CK(cudaEventCreateWithFlags(&c->ev_join[1], cudaEventDisableTiming));
   CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&c->ev_u, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->ev_u_fork, cudaEventDisableTiming));
@@ -506,11 +486,6 @@ int echo_gpu_free(EchoCtx* c) {
   echo_hyp_free(c->hyp);
   echo_out_free(c);
   cudaStreamDestroy(c->stream);
-  cudaStreamDestroy(c->side[0]);
-  cudaStreamDestroy(c->side[1]);
-  cudaEventDestroy(c->ev_fork);
-  cudaEventDestroy(c->ev_join[0]);
-  cudaEventDestroy(c->ev_join[1]);
   cudaStreamDestroy(c->copy_stream);
   cudaEventDestroy(c->ev_u);
   cudaEventDestroy(c->ev_u_fork);
@@ -1070,10 +1045,7 @@ int echo_gpu_rhs(EchoCtx* c, double* du, double* amax3) {
   size_t nvc = (size_t)c->nv * c->g.ncell;
   if (!c->d_du) CK(cudaMalloc(&c->d_du, sizeof(double) * nvc));
   CK(cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream));
-  for (int d = 0; d < 3; d++) {
-    int n = d == 0 ? c->g.nx : d == 1 ? c->g.ny : c->g.nz;
-    if (n > 1) DISPATCH(c, launch_faces, c, d);
-  }
+  launch_sweeps(c);
   DISPATCH(c, launch_update, c, 1, MODE_RHS, c->d_du);
   CK(cudaGetLastError());
   if (du) CK(cudaMemcpyAsync(du, c->d_du, sizeof(double) * nvc, cudaMemcpyDeviceToHost, c->stream));

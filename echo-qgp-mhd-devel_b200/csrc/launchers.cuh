@@ -10,45 +10,55 @@ namespace echo {
 // ---------------------------------------------------------------------------
 // kernel dispatch
 // ---------------------------------------------------------------------------
+// Tile of the sweeps (faces.cuh): 256 cells, one thread each, where that
+// fills the device; smaller tiles, with the block's further threads sharing the
+// variables, where it does not.
+inline int sweep_lc(const EchoCtx* c, int mask) {
+  unsigned t = 0;
+  for (int d = 0; d < 3; d++)
+    if (mask >> d & 1) t += tiles_of(c->g, d, 8, 4);
+  return t >= 2 * 148 ? 8 : 5;
+}
+
+// the sweeps of the directions in mask (bit d: direction d), one launch
 template <int KIND>
-void launch_faces(EchoCtx* c, int dir) {
-  FaceArgs A;
-  A.P = c->P;
-  A.g = c->g;
-  A.bc = c->bc[dir];
-  A.bc_uniform = c->bc_uniform[dir];
-  A.bc_signed = c->bc_signed[dir];
-  A.v = c->d_v[c->vcur];
-  A.F = c->d_F[dir];
-  A.WD = c->d_WD[dir];
-  A.sc = c->d_sc;
-  A.coordinates = c->p.coordinates;
-  unsigned blocks = (unsigned)((c->nfaces[dir] + 127) / 128);
-#ifndef ECHO_EXACT
-  // product build: the cell-centred sweep in segments of face_mode cells
-  if (c->p.recal == ECHO_REC_WENO5 && c->face_mode > 0) {
-    const Grid& g = c->g;
-    if (c->face_mode == 8) {
-      if (dir == 0) faces_seg_kernel<KIND, 0, 8><<<(unsigned)((seg_warps<0, 8>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-      if (dir == 1) faces_seg_kernel<KIND, 1, 8><<<(unsigned)((seg_warps<1, 8>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-      if (dir == 2) faces_seg_kernel<KIND, 2, 8><<<(unsigned)((seg_warps<2, 8>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-    } else {
-      if (dir == 0) faces_seg_kernel<KIND, 0, 16><<<(unsigned)((seg_warps<0, 16>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-      if (dir == 1) faces_seg_kernel<KIND, 1, 16><<<(unsigned)((seg_warps<1, 16>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-      if (dir == 2) faces_seg_kernel<KIND, 2, 16><<<(unsigned)((seg_warps<2, 16>(g) + 3) / 4), 128, 0, c->stream>>>(A);
-    }
-    return;
+void launch_faces(EchoCtx* c, int mask) {
+  SweepArgs S;
+  memset(&S, 0, sizeof(S));
+  // pencils of a tile of the y and eta sweeps: 16, or as many as leave
+  // face_mode cells of each in a tile (echo_gpu_set_faces)
+  const int lc = sweep_lc(c, mask);
+  S.lw = c->face_mode == 8 ? lc - 3 : c->face_mode == 16 || lc == 8 ? lc - 4 : lc - 3;
+  unsigned blocks = 0;
+  for (int d = 0; d < 3; d++) {
+    S.first[d] = blocks;
+    FaceArgs& A = S.A[d];
+    A.P = c->P;
+    A.g = c->g;
+    A.bc = c->bc[d];
+    A.bc_uniform = c->bc_uniform[d];
+    A.bc_signed = c->bc_signed[d];
+    A.v = c->d_v[c->vcur];
+    A.F = c->d_F[d];
+    A.WD = c->d_WD[d];
+    A.sc = c->d_sc;
+    A.coordinates = c->p.coordinates;
+    if (mask >> d & 1) blocks += tiles_of(c->g, d, lc, S.lw);
   }
-#endif
-  if (c->p.recal == ECHO_REC_WENO5) {
-    if (dir == 0) faces_kernel<KIND, 0, ECHO_REC_WENO5><<<blocks, 128, 0, c->stream>>>(A);
-    if (dir == 1) faces_kernel<KIND, 1, ECHO_REC_WENO5><<<blocks, 128, 0, c->stream>>>(A);
-    if (dir == 2) faces_kernel<KIND, 2, ECHO_REC_WENO5><<<blocks, 128, 0, c->stream>>>(A);
-  } else {
-    if (dir == 0) faces_kernel<KIND, 0, REC_RUNTIME><<<blocks, 128, 0, c->stream>>>(A);
-    if (dir == 1) faces_kernel<KIND, 1, REC_RUNTIME><<<blocks, 128, 0, c->stream>>>(A);
-    if (dir == 2) faces_kernel<KIND, 2, REC_RUNTIME><<<blocks, 128, 0, c->stream>>>(A);
-  }
+  S.first[3] = blocks;
+  const size_t smem = tile_smem<KIND>(lc);
+  auto go = [&](auto* fn) {
+    if (smem > 40 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    fn<<<blocks, ECHO_SWEEP_NT, smem, c->stream>>>(S);
+  };
+  // the schemes in use get a kernel of their own; the others choose at run time
+  auto pick = [&](auto big, auto small) { lc == 8 ? go(big) : go(small); };
+  if (c->p.recal == ECHO_REC_WENO5)
+    pick(sweep_kernel<KIND, ECHO_REC_WENO5, 8>, sweep_kernel<KIND, ECHO_REC_WENO5, 5>);
+  else if (c->p.recal == ECHO_REC_MPE5)
+    pick(sweep_kernel<KIND, ECHO_REC_MPE5, 8>, sweep_kernel<KIND, ECHO_REC_MPE5, 5>);
+  else
+    pick(sweep_kernel<KIND, REC_RUNTIME, 8>, sweep_kernel<KIND, REC_RUNTIME, 5>);
 }
 
 template <int KIND>

@@ -168,15 +168,15 @@ extern "C" int echo_gpu_rhs_noalloc(const EchoParams* p, const double* d_eos_col
   (void)cudaGetLastError();
   double g3 = p->coordinates == ECHO_BJORKEN ? t * t : 1.;
   noalloc_reset_scalars<<<1, 1, 0, c.stream>>>(c.d_sc, t, pow(t, 3.), g3);
-  for (int d = 0; d < 3; d++) {
-    if (n[d] <= 1) continue;
-    switch (kind) {
-      case KIND_HD: launch_faces<KIND_HD>(&c, d); break;
-      case KIND_VISC: launch_faces<KIND_VISC>(&c, d); break;
-      case KIND_MHD: launch_faces<KIND_MHD>(&c, d); break;
-      default: launch_faces<KIND_MHDGLM>(&c, d); break;
+  int mask = 0;
+  for (int d = 0; d < 3; d++)
+    if (n[d] > 1) mask |= 1 << d;
+  if (mask) switch (kind) {
+      case KIND_HD: launch_faces<KIND_HD>(&c, mask); break;
+      case KIND_VISC: launch_faces<KIND_VISC>(&c, mask); break;
+      case KIND_MHD: launch_faces<KIND_MHD>(&c, mask); break;
+      default: launch_faces<KIND_MHDGLM>(&c, mask); break;
     }
-  }
   switch (kind) {
     case KIND_HD: launch_update<KIND_HD>(&c, 1, MODE_RHS, d_du); break;
     case KIND_VISC: launch_update<KIND_VISC>(&c, 1, MODE_RHS, d_du); break;

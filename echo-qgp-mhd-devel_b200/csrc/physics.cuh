@@ -125,6 +125,36 @@ __device__ __forceinline__ double over_gp(const Metric& M, double x) {
 #endif
 }
 
+#ifndef ECHO_EXACT
+// ---------------------------------------------------------------------------
+// Reciprocal, reciprocal square root and square root of the product build:
+// the hardware's approximation (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64)
+// and one third-order Householder correction each (Householder, The Numerical
+// Treatment of a Single Nonlinear Equation, 1970, ch. 4: x (1 + e + e^2) for
+// 1/a with e = 1 - a x, y (1 + e/2 + 3 e^2 / 8) for 1/sqrt(a) with
+// e = 1 - a y^2), without the special-case branches of the division and of
+// sqrt().  For normal a whose reciprocal is normal too; the callers' operands
+// are (denominators of the WENO weights, 1 - v^2, wave-speed sums).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double rcp_h3(double a) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  const double e = fma(-a, x, 1.);
+  return fma(x, fma(e, e, e), x);
+}
+__device__ __forceinline__ double rsqrt_h3(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  const double e = fma(-a * y, y, 1.);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+// sqrt(a); arguments below 1e-290 (zero: a state without sound) give 0
+__device__ __forceinline__ double sqrt_h3(double a) {
+  const double r = a * rsqrt_h3(a);
+  return fabs(a) < 1e-290 ? 0. : r;
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // equation of state (eos.f90)
 // ---------------------------------------------------------------------------
@@ -385,82 +415,69 @@ __device__ __forceinline__ double mp5(double f, double f1, double f2, double f3,
 
 // WENO5 one side: f1..f5 in the reference's naming (holib.f90:198-212)
 #ifndef ECHO_EXACT
-// Product build: the same weights with the common denominator multiplied
-// through, sum_k d_k p_k / q_k^2 / sum_k d_k / q_k^2 =
-// sum_k d_k p_k Q_j Q_l / sum_k d_k Q_j Q_l with Q = q^2 (Q >= 1e-12, so
-// the products cannot underflow), and the two sides of a face sharing one
-// division: gl = nl/dl, gr = nr/dr = (nl dr, nr dl) / (dl dr), where
-// dl, dr >= 3e-24 and stay far below 1e150 for the values a run holds.
-__device__ __forceinline__ void weno5_nd(double f1, double f2, double f3, double f4, double f5, double& num,
-                                         double& den) {
-  // The smoothness indicators beta_k / 12 + eps = 13/12 t1^2 + 1/4 t2^2 + eps
-  // as two fused multiply-adds each, the sub-stencil polynomials with the
-  // factor 1/8 and the linear weights 10 and 5 of p2 and p3 folded into their
-  // (exactly representable) coefficients, and the denominator sum_k d_k Q_j Q_l
-  // with d = (1, 10, 5): the same weights with fewer FP64 instructions.
-  const double eps = 1.e-6, c13 = 13. / 12.;
-  double t1, t2, q1, q2, q3;
-  t1 = f3 - 2 * f2 + f1;
-  t2 = fma(3., f3, fma(-4., f2, f1));
-  q1 = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
-  t1 = f4 - 2 * f3 + f2;
-  t2 = f4 - f2;
-  q2 = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
-  t1 = f5 - 2 * f4 + f3;
-  t2 = fma(3., f3, fma(-4., f4, f5));
-  q3 = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
-  double Q1 = q1 * q1, Q2 = q2 * q2, Q3 = q3 * q3;
-  double w1 = Q2 * Q3, w2 = Q1 * Q3, w3 = Q1 * Q2;
-  double p1 = fma(1.875, f3, fma(-1.25, f2, 0.375 * f1));       // (3 f1 - 10 f2 + 15 f3) / 8
-  double p2 = fma(3.75, f4, fma(7.5, f3, -1.25 * f2));          // 10 (-f2 + 6 f3 + 3 f4) / 8
-  double p3 = fma(-0.625, f5, fma(3.75, f4, 1.875 * f3));       // 5 (3 f3 + 6 f4 - f5) / 8
-  num = fma(w3, p3, fma(w2, p2, w1 * p1));
-  den = fma(5., w3, fma(10., w2, w1));
+// Product build: the scheme in differences of neighbouring values.  With
+// d_i the first and D_i the second differences of a side's stencil f1..f5,
+// 4 (beta_k / 12 + eps) is 13/3 D^2 + t^2 + 4 eps with t = 2 d + D, d + d or
+// D - 2 d; the sub-stencil polynomials are f3 + delta_k with delta_k two terms
+// in d (below, the factor 1/8 and the linear weights 10 and 5 folded into
+// their exactly representable coefficients).  The common denominator of the
+// weights is multiplied through, sum_k d_k delta_k / q_k^2 / sum_k d_k / q_k^2
+// = sum_k d_k delta_k Q_j Q_l / sum_k d_k Q_j Q_l with Q = q^2 (q >= 4e-6, so
+// the products cannot underflow), and the two states share one reciprocal:
+// n1/m1 and n2/m2 = (n1 m2, n2 m1) / (m1 m2), where m1, m2 >= 1e-21 and stay
+// far below 1e150 for the values a run holds.  The difference form needs 56
+// FP64 instructions for both states of a cell (the same in values: 101 for the
+// two states of a face) and rounds less: the cancellations of nearly equal
+// values are the exact differences d_i.
+__device__ __forceinline__ double weno5_q(double D, double t) {  // 4 (beta / 12 + eps)
+  return fma(t, t, fma((13. / 3.) * D, D, 4.e-6));
 }
-// Cell-centred WENO5 (product build): both face states of one cell from its
-// five-point stencil f1..f5 = v(c-2..c+2).  plus = the state at c+1/2 (the
-// left state of the face above, holib.f90:198-212 on f1..f5), minus = the
-// state at c-1/2 (the right state of the face below, the same formula on
-// f5..f1).  The two orientations share their three smoothness indicators
-// (the reversed stencil's first is the forward stencil's third) and the
-// three products of the weights, and one division serves both.
+// numerator (without f3) and denominator of a side from its first differences
+// and the products w1 = Q2 Q3, w2 = Q1 Q3, w3 = Q1 Q2
+__device__ __forceinline__ void weno5_nm(double d0, double d1, double d2, double d3, double w1, double w2, double w3,
+                                         double& n, double& m) {
+  const double e1 = fma(0.875, d1, -0.375 * d0);   // (7 d1 - 3 d0) / 8
+  const double e2 = fma(3.75, d2, 1.25 * d1);      // 10 (3 d2 + d1) / 8
+  const double e3 = fma(3.125, d2, -0.625 * d3);   // 5 (5 d2 - d3) / 8
+  n = fma(w3, e3, fma(w2, e2, w1 * e1));
+  m = fma(5., w3, fma(10., w2, w1));
+}
+// Both face states of one cell from its five-point stencil f1..f5 =
+// v(c-2..c+2): plus = the state at c+1/2 (the left state of the face above,
+// holib.f90:198-212 on f1..f5), minus = the state at c-1/2 (the right state of
+// the face below, the same formula on f5..f1).  The two orientations share
+// their three smoothness indicators.
 __device__ __forceinline__ void weno5_cell(double f1, double f2, double f3, double f4, double f5, double& plus,
                                            double& minus) {
-  const double eps = 1.e-6, c13 = 13. / 12.;
-  double t1, t2;
-  t1 = f3 - 2 * f2 + f1;
-  t2 = fma(3., f3, fma(-4., f2, f1));
-  const double qa = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
-  t1 = f4 - 2 * f3 + f2;
-  t2 = f4 - f2;
-  const double qb = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
-  t1 = f5 - 2 * f4 + f3;
-  t2 = fma(3., f3, fma(-4., f4, f5));
-  const double qc = fma(c13 * t1, t1, fma(0.25 * t2, t2, eps));
+  const double d0 = f2 - f1, d1 = f3 - f2, d2 = f4 - f3, d3 = f5 - f4;
+  const double Da = d1 - d0, Db = d2 - d1, Dc = d3 - d2;
+  const double qa = weno5_q(Da, fma(2., d1, Da)), qb = weno5_q(Db, d1 + d2), qc = weno5_q(Dc, fma(-2., d2, Dc));
   const double Qa = qa * qa, Qb = qb * qb, Qc = qc * qc;
   const double wbc = Qb * Qc, wac = Qa * Qc, wab = Qa * Qb;
-  // forward: weights (wbc, 10 wac, 5 wab); reversed: (wab, 10 wac, 5 wbc)
-  const double p1 = fma(1.875, f3, fma(-1.25, f2, 0.375 * f1));
-  const double p2 = fma(3.75, f4, fma(7.5, f3, -1.25 * f2));
-  const double p3 = fma(-0.625, f5, fma(3.75, f4, 1.875 * f3));
-  const double r1 = fma(1.875, f3, fma(-1.25, f4, 0.375 * f5));
-  const double r2 = fma(3.75, f2, fma(7.5, f3, -1.25 * f4));
-  const double r3 = fma(-0.625, f1, fma(3.75, f2, 1.875 * f3));
-  const double np = fma(wab, p3, fma(wac, p2, wbc * p1));
-  const double dp = fma(5., wab, fma(10., wac, wbc));
-  const double nm = fma(wbc, r3, fma(wac, r2, wab * r1));
-  const double dm = fma(5., wbc, fma(10., wac, wab));
-  const double inv = 1. / (dp * dm);
-  plus = np * dm * inv;
-  minus = nm * dp * inv;
+  double np, mp, nm, mm;
+  weno5_nm(d0, d1, d2, d3, wbc, wac, wab, np, mp);
+  weno5_nm(d3, d2, d1, d0, wab, wac, wbc, nm, mm);  // reversed: the differences change sign
+  const double inv = rcp_h3(mp * mm);
+  plus = fma(np * mm, inv, f3);
+  minus = fma(-nm * mp, inv, f3);
 }
+// Left and right state of the face between s[2] and s[3]
 __device__ __forceinline__ void weno5_face(const double s[6], double& gl, double& gr) {
-  double nl, dl, nr, dr;
-  weno5_nd(s[0], s[1], s[2], s[3], s[4], nl, dl);
-  weno5_nd(s[5], s[4], s[3], s[2], s[1], nr, dr);
-  double inv = 1. / (dl * dr);
-  gl = nl * dr * inv;
-  gr = nr * dl * inv;
+  const double d0 = s[1] - s[0], d1 = s[2] - s[1], d2 = s[3] - s[2], d3 = s[4] - s[3], d4 = s[5] - s[4];
+  const double D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3;
+  double q1 = weno5_q(D1, fma(2., d1, D1)), q2 = weno5_q(D2, d1 + d2), q3 = weno5_q(D3, fma(-2., d2, D3));
+  double Q1 = q1 * q1, Q2 = q2 * q2, Q3 = q3 * q3, nl, ml, nr, mr;
+  weno5_nm(d0, d1, d2, d3, Q2 * Q3, Q1 * Q3, Q1 * Q2, nl, ml);
+  q1 = weno5_q(D4, fma(-2., d3, D4));
+  q2 = weno5_q(D3, d2 + d3);
+  q3 = weno5_q(D2, fma(2., d2, D2));
+  Q1 = q1 * q1;
+  Q2 = q2 * q2;
+  Q3 = q3 * q3;
+  weno5_nm(d4, d3, d2, d1, Q2 * Q3, Q1 * Q3, Q1 * Q2, nr, mr);
+  const double inv = rcp_h3(ml * mr);
+  gl = fma(nl * mr, inv, s[2]);
+  gr = fma(-nr * ml, inv, s[3]);
 }
 #else
 __device__ __forceinline__ double weno5_side(double f1, double f2, double f3, double f4, double f5) {
@@ -575,6 +592,57 @@ enum { REC_RUNTIME = -1 };
 template <int REC>
 __device__ __forceinline__ void recon_face(int recal, const double s[6], double& gl, double& gr) {
   recon_any(REC >= 0 ? REC : recal, s, gl, gr);
+}
+
+// Both face states of the cell f[2] from its five-point stencil: plus as
+// recon_any's left state of the face above it, minus as its right state of
+// the face below (the same expressions, so the parity build's bits).
+template <int REC>
+__device__ __forceinline__ void recon_cell(int recal, const double f[5], double& plus, double& minus) {
+  switch (REC >= 0 ? REC : recal) {
+    case ECHO_REC_TVD2: {
+      const double h = .5 * mm2(f[2] - f[1], f[3] - f[2]);
+      plus = f[2] + h;
+      minus = f[2] - h;
+      break;
+    }
+    case ECHO_REC_CENO3:
+      plus = ceno3_side(f[0], f[1], f[2], f[3], f[4]);
+      minus = ceno3_side(f[4], f[3], f[2], f[1], f[0]);
+      break;
+    case ECHO_REC_WENO3:
+      plus = weno3_side(f[1], f[2], f[3]);
+      minus = weno3_side(f[3], f[2], f[1]);
+      break;
+    case ECHO_REC_WENO5:
+#ifdef ECHO_EXACT
+      plus = weno5_side(f[0], f[1], f[2], f[3], f[4]);
+      minus = weno5_side(f[4], f[3], f[2], f[1], f[0]);
+#else
+      weno5_cell(f[0], f[1], f[2], f[3], f[4], plus, minus);
+#endif
+      break;
+    case ECHO_REC_PPM4:
+      plus = ppm4_side(f[1], f[2], f[3], f[4]);
+      minus = ppm4_side(f[3], f[2], f[1], f[0]);
+      break;
+    case ECHO_REC_MPE3: {
+      const double d1 = -1 / 8., d2 = 6 / 8., d3 = 3 / 8.;
+      double l = d1 * f[1] + d2 * f[2] + d3 * f[3];
+      double r = d1 * f[3] + d2 * f[2] + d3 * f[1];
+      plus = mp5(l, f[0], f[1], f[2], f[3], f[4]);
+      minus = mp5(r, f[4], f[3], f[2], f[1], f[0]);
+      break;
+    }
+    default: {  // MPE5
+      const double d1 = 3 / 128., d2 = -20 / 128., d3 = 90 / 128., d4 = 60 / 128., d5 = -5 / 128.;
+      double l = d1 * f[0] + d2 * f[1] + d3 * f[2] + d4 * f[3] + d5 * f[4];
+      double r = d1 * f[4] + d2 * f[3] + d3 * f[2] + d4 * f[1] + d5 * f[0];
+      plus = mp5(l, f[0], f[1], f[2], f[3], f[4]);
+      minus = mp5(r, f[4], f[3], f[2], f[1], f[0]);
+      break;
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------

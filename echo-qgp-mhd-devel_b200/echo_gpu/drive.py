@@ -60,8 +60,8 @@ def main():
                     help="fused stage kernel or the sweep kernels (auto: the library's default)")
     ap.add_argument("--tile", default="", help="fused stage tile tx,ty,zseg (0 = chosen for the grid)")
     ap.add_argument("--faces", type=int, default=-1, choices=[-1, 0, 8, 16],
-                    help="product build face sweeps: 0 one thread per face, 8/16 cell-centred segments "
-                         "(-1: the library's default)")
+                    help="product build face sweeps: 8/16 cells along a y or eta tile, 0 the library's choice "
+                         "(-1: leave it)")
     a = ap.parse_args()
     if a.config == "batch":
         run_batch(a)

@@ -303,14 +303,13 @@ class Evolve:
         return {k: (float(ms[i]), int(n[i])) for i, k in enumerate(self.KERNEL_CLASSES)}
 
     def set_faces(self, mode: int):
-        """Product build: how the WENO5 face sweeps run -- 0 one thread per
-        face (the default), 8 or 16 cell-centred segments of that many
-        cells."""
+        """Product build: cells along the sweep of a y or eta tile -- 0 the
+        library's choice (the default), 8 or 16."""
         self._check(self.lib.echo_gpu_set_faces(self.h, mode), "set_faces")
 
     def set_sweeps(self, concurrent: bool = True):
-        """The x, y and eta sweeps of a stage side by side on three streams
-        (the default) or one after another."""
+        """The x, y and eta sweeps of a stage in one launch (the default) or
+        one after another."""
         self._check(self.lib.echo_gpu_set_sweeps(self.h, int(concurrent)), "set_sweeps")
 
     def set_stage(self, fused: bool = True, tx: int = 0, ty: int = 0, zseg: int = 0) -> dict:

@@ -344,26 +344,21 @@ int echo_gpu_hyp_get(EchoCtx* ctx, double* out);
  * run. */
 int echo_gpu_profile_step(EchoCtx* ctx, double* ms, int* launches);
 
-/* No counterpart in the reference (an execution option).  How the product
- * build (libechogpu.so) computes the WENO5 face sweeps:
- *   mode 0   one thread per face, both face states in one thread (the
- *            default; the reference's arrangement, which the parity build
- *            always runs);
- *   mode 8, 16  one thread per cell, in segments of that many cells along
- *            the sweep: a thread reconstructs both face states of its cell
- *            from one set of WENO5 smoothness indicators and takes the
- *            state of the cell below from its neighbouring lane, so a
- *            segment yields mode - 1 faces.
- * All meet the oracle at the product build's tolerance.  Other
- * reconstructions always run mode 0.  ECHO_ERR_ARG for other modes.
- * Synchronises the stream and drops the step graphs. */
+/* No counterpart in the reference (an execution option).  The face sweeps
+ * reconstruct each cell's two face states once, a block on a tile of cells
+ * (csrc/faces.cuh).  How many cells a y or eta tile has along the sweep, in
+ * the product build (libechogpu.so):
+ *   mode 0   the library's choice for the grid (the default; the parity
+ *            build always runs it);
+ *   mode 8, 16  that many; a tile yields one face fewer along the sweep.
+ * A face's arithmetic does not depend on the tile.  ECHO_ERR_ARG for other
+ * modes.  Synchronises the stream and drops the step graphs. */
 int echo_gpu_set_faces(EchoCtx* ctx, int mode);
 
 /* No counterpart in the reference (an execution option).  concurrent = 1
- * (the default) runs the x, y and eta flux sweeps of a stage side by side
- * on three streams, joined before the update; 0 runs them one after
- * another.  The sweeps are independent, so both give the same bits.
- * Synchronises the stream and drops the step graphs. */
+ * (the default) runs the x, y and eta flux sweeps of a stage in one launch;
+ * 0 runs them one after another.  The sweeps are independent, so both give
+ * the same bits.  Synchronises the stream and drops the step graphs. */
 int echo_gpu_set_sweeps(EchoCtx* ctx, int concurrent);
 
 /* No counterpart in the reference (an execution option).  How a stage runs:
