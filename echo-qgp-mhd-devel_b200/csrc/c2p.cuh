@@ -16,6 +16,29 @@ struct Sist3 {
   double iUB;  // 1 / (|U| + B2), the scale of the second residual
 };
 
+#ifndef ECHO_EXACT
+// at: the EoS interval of the last evaluation (the finite differences of
+// BRENTM hardly move p)
+__device__ __forceinline__ double sist3_f(const DevPhys& P, const Sist3& s, const double* X, int K, EosAt& at) {
+  const double xx = X[0], yy = X[1], pp = X[2];
+  if (K == 3) {
+    double en = 0;
+    if (P.eqstate == ECHO_EOS_TABLE && P.rec) {  // an error leaves en = 0 (system.f90:1227)
+      if (!eos_holds(at, at.p0, pp)) {
+        at.h = 0;
+        if (!(pp < P.pmin) && !(pp > P.pmax)) eos_at_p(P, pp, at);
+      }
+      if (at.h) en = at.e0 + (pp - at.p0) * at.sl;
+    } else {
+      (void)eos_energy(P, s.D * sqrt(1 - xx), &en, pp);
+    }
+    return yy - (pp + en) * rcp_h3(1 - xx);
+  }
+  const double iy = rcp_h3(yy), q = s.SB2 * (iy * iy);
+  if (K == 1) return (yy + s.B2) * (yy + s.B2) * xx - q * (2 * yy + s.B2) - s.S2;
+  return yy - pp + 0.5 * (1. + xx) * s.B2 - 0.5 * q - s.U;
+}
+#else
 __device__ __forceinline__ double sist3_f(const DevPhys& P, const Sist3& s, const double* X, int K) {
   double xx = X[0], yy = X[1], pp = X[2];
   if (K == 1) return (yy + s.B2) * (yy + s.B2) * xx - s.SB2 / (yy * yy) * (2 * yy + s.B2) - s.S2;
@@ -24,6 +47,7 @@ __device__ __forceinline__ double sist3_f(const DevPhys& P, const Sist3& s, cons
   (void)eos_energy(P, rh, &en, pp);  // errcode ignored (system.f90:1227)
   return yy - (pp + en) / (1 - xx);
 }
+#endif
 
 __device__ __forceinline__ double dmax1(double a, double b) { return b > a ? b : a; }
 
@@ -182,12 +206,24 @@ static __device__ int brentm(Sys& sys, double* X, double FTOL, double XTOL, int 
 struct Sist3F {
   const DevPhys& P;
   const Sist3& s;
+#ifdef ECHO_EXACT
   __device__ double f(const double* X, int K) const { return sist3_f(P, s, X, K); }
+#else
+  EosAt at;
+  __device__ __forceinline__ double f(const double* X, int K) { return sist3_f(P, s, X, K, at); }
+#endif
 };
 static __device__ int brentm3(const DevPhys& P, const Sist3& s, double* X, double FTOL, double XTOL, int MAXFEV,
                               int MOPT, int* nfev_out) {
   Sist3F sys{P, s};
+#ifndef ECHO_EXACT
+  sys.at.h = 0;
+#endif
   return brentm<3>(sys, X, FTOL, XTOL, MAXFEV, MOPT, nfev_out);
+}
+// out of line, for the kernels that solve by Newton
+static __device__ __noinline__ int brentm3_call(const DevPhys& P, const Sist3& s, double* X, int* nfev_out) {
+  return brentm3(P, s, X, 1.e-14, 1.e-14, 300, 3, nfev_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -434,7 +470,7 @@ static __device__ __noinline__ int cons2prim_mhd_algo(const DevPhys& P, const Me
     double B2 = bx * bx + by * by + bz * bz * g3;
     double SB = sx * bx + sy * by + sz * bz;
     double SB2 = SB * SB;
-    double SS2 = sx * sx + sy * sy + sz * sz / g3;
+    double SS2 = sx * sx + sy * sy + over_g3(M, sz * sz);
     double rh = v[KRH], vx = v[KVX], vy = v[KVY], vz = v[KVZ], pr = v[KPR], en = 0;
     errcode = eos_energy(P, rh, &en, pr);
     double xs, ys;
@@ -647,14 +683,6 @@ __device__ __forceinline__ int eos_energy_slope(const DevPhys& P, double rh, dou
     if (pr < __ldg(P.tp)) return 125;
     if (pr > __ldg(P.tp + P.nt - 1)) return 126;
     int h = SEARCH_P(P, pr);
-#ifndef ECHO_EXACT
-    if (P.sl_ep) {
-      double sl = __ldg(P.sl_ep + h - 2);
-      *dedp = sl;
-      *en = __ldg(P.te + h - 2) + (pr - __ldg(P.tp + h - 2)) * sl;
-      return 0;
-    }
-#endif
     double p2 = __ldg(P.tp + h - 1), p1 = __ldg(P.tp + h - 2);
     double e2 = __ldg(P.te + h - 1), e1 = __ldg(P.te + h - 2);
     *dedp = (e2 - e1) / (p2 - p1);
@@ -676,10 +704,79 @@ __device__ __forceinline__ int eos_energy_slope(const DevPhys& P, double rh, dou
   return 0;
 }
 
+#ifndef ECHO_EXACT
+// the same from the interval of the last call where that still holds pr
+__device__ __forceinline__ int eos_energy_slope_at(const DevPhys& P, double rh, double pr, double* en, double* dedp,
+                                                   EosAt& a) {
+  if (P.eqstate != ECHO_EOS_TABLE || !P.rec) return eos_energy_slope(P, rh, pr, en, dedp);
+  if (!eos_holds(a, a.p0, pr)) {
+    if (pr < P.pmin) return 125;
+    if (pr > P.pmax) return 126;
+    eos_at_p(P, pr, a);
+  }
+  *dedp = a.sl;
+  *en = a.e0 + (pr - a.p0) * a.sl;
+  return 0;
+}
+#endif
+
 // Newton on sist3 with the analytic Jacobian.  Converged when the relative
 // residual max(|F1|/(y+B^2)^2, |F2|/(|U|+B^2), |F3|/y) <= tol; one more
 // Newton correction is then applied (the error after it is ~ residual^2).
 // Returns the number of corrections made, or -1 (the caller falls back).
+#ifndef ECHO_EXACT
+// Product build: the same Newton with the third unknown eliminated.  The
+// second equation gives dp = F2 + J21 dx + J22 dy (J23 = -1), the third then
+// A dx + B dy = R; with the first that is a 2 x 2 system.  Three reciprocals
+// a step (y, 1 - x, the determinant); the residual test multiplies by the
+// scales instead of dividing.
+static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, double tol, int maxit) {
+  double xx = X[0], yy = X[1], pp = X[2];
+  EosAt at;
+  at.h = 0;
+  for (int it = 0; it <= maxit; it++) {
+    if (!(xx < 1.0) || !(xx >= 0.0) || !(yy > 0.0) || !(pp > 0.0)) return -1;
+    double en = 0, dedp = 0;
+    const double rh = P.eqstate == ECHO_EOS_IDEALGAS ? s.D * sqrt(1. - xx) : 0.;  // e depends on rho there only
+    if (eos_energy_slope_at(P, rh, pp, &en, &dedp, at)) return -1;
+    const double ib = yy + s.B2, ib2 = ib * ib, iy = rcp_h3(yy), i1x = rcp_h3(1. - xx);
+    const double q2 = s.SB2 * (iy * iy), q3 = q2 * iy;
+    const double F1 = ib2 * xx - q2 * (2 * yy + s.B2) - s.S2;
+    const double F2 = yy - pp + 0.5 * (1. + xx) * s.B2 - 0.5 * q2 - s.U;
+    const double F3 = yy - (pp + en) * i1x;
+    const bool done = fabs(F1) <= tol * ib2 && fabs(F2) * s.iUB <= tol && fabs(F3) * iy <= tol;
+    const double J12 = 2 * (ib * xx + q3 * (2 * yy + s.B2) - q2), J21 = 0.5 * s.B2, J22 = 1. + q3;
+    const double J31 = -(pp + en) * (i1x * i1x), J33 = -(1. + dedp) * i1x;
+    const double A = J31 + J33 * J21, B = 1. + J33 * J22, R = -(F3 + J33 * F2);
+    const double det = ib2 * B - J12 * A;
+    if (det == 0.0 || !isfinite(det)) return -1;
+    const double idet = rcp_h3(det);
+    const double dx = -(F1 * B + J12 * R) * idet, dy = (ib2 * R + F1 * A) * idet;
+    const double dp = F2 + J21 * dx + J22 * dy;
+    if (done) {  // converged: polish and stop
+      xx += dx;
+      yy += dy;
+      pp += dp;
+      if (!(xx < 1.0) || !(yy > 0.0) || !(pp > 0.0)) return -1;
+      X[0] = xx;
+      X[1] = yy;
+      X[2] = pp;
+      return it + 1;
+    }
+    if (it == maxit) return -1;
+    // damp steps that would leave the physical domain
+    double lam = 1.0;
+    for (int k = 0; k < 30 && (xx + lam * dx >= 1.0 || xx + lam * dx < 0.0 || yy + lam * dy <= 0.0 ||
+                               pp + lam * dp <= 0.0);
+         k++)
+      lam *= 0.5;
+    xx += lam * dx;
+    yy += lam * dy;
+    pp += lam * dp;
+  }
+  return -1;
+}
+#else
 static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, double tol, int maxit) {
   double xx = X[0], yy = X[1], pp = X[2];
   for (int it = 0; it <= maxit; it++) {
@@ -691,14 +788,8 @@ static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, doubl
     double F1 = ib * ib * xx - s.SB2 * iy2 * (2 * yy + s.B2) - s.S2;
     double F2 = yy - pp + 0.5 * (1. + xx) * s.B2 - 0.5 * s.SB2 * iy2 - s.U;
     double F3 = yy - (pp + en) * i1x;
-#ifdef ECHO_EXACT
     double iy3 = iy2 / yy;
     double r = fmax(fabs(F1) / (ib * ib), fmax(fabs(F2) / (fabs(s.U) + s.B2), fabs(F3) / yy));
-#else
-    // 1/y = y * (1/y^2); the residual scales as reciprocals (one division)
-    double iy1 = yy * iy2, iy3 = iy2 * iy1;
-    double r = fmax(fabs(F1) / (ib * ib), fmax(fabs(F2) * s.iUB, fabs(F3) * iy1));
-#endif
     // d(en)/dx through rh is zero: the tabulated and conformal e(p) do not depend on rh
     double J11 = ib * ib, J12 = 2 * ib * xx + 2 * s.SB2 * (2 * yy + s.B2) * iy3 - 2 * s.SB2 * iy2, J13 = 0.;
     double J21 = 0.5 * s.B2, J22 = 1. + s.SB2 * iy3, J23 = -1.;
@@ -735,6 +826,61 @@ static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, doubl
   }
   return -1;
 }
+#endif
+
+// The Newton step on p of the ideal-hydro inversion (system.f90:511-561), for
+// e = w (1 - v^2) - p - extra with w = et + p.  An EoS lookup out of range
+// leaves pe and its derivatives as the step before left them.
+struct FluidNewton {
+  EosAt at;
+  double pe, dprdrh, dprden;
+  __device__ __forceinline__ FluidNewton() : pe(0.), dprdrh(0.), dprden(0.) { at.h = 0; }
+};
+// One step: the state it is taken at (w, v^2 and, parity build, rho) and the
+// correction dpr.  Returns true when v^2 >= 1 (dpr is not set then).
+__device__ __forceinline__ bool fluid_step(const DevPhys& P, double d, double s2, double et, double extra, double pr,
+                                           FluidNewton& n, double& w, double& v2, double& rh, double& dpr,
+                                           int& errcode) {
+  w = et + pr;
+#ifdef ECHO_EXACT
+  v2 = s2 / (w * w);
+  if (v2 >= 1.) return true;
+  const double glf = 1. / sqrt(1. - v2);
+  rh = d / glf;
+  const double en = w * (1. - v2) - pr - extra;
+  const double drhdpr = rh * v2 * glf / (en + pr), dendpr = v2;
+  errcode = eos_pressure(P, rh, en, &n.pe, &n.dprdrh, &n.dprden);
+  const double f = n.pe - pr, df = n.dprdrh * drhdpr + n.dprden * dendpr - 1.;
+  dpr = -f / df;
+#else
+  // two reciprocals a step (w, the derivative) and no square root: rho enters
+  // p only through dp/drho, which is zero but for the ideal gas; the callers
+  // take it after the last step (fluid_rho)
+  const double rw = rcp_h3(w);
+  v2 = s2 * (rw * rw);
+  if (v2 >= 1. || w == 0.) {
+    v2 = 1.;
+    return true;
+  }
+  const double i1 = 1. - v2, en = w * i1 - pr - extra;
+  double df;
+  if (P.eqstate == ECHO_EOS_IDEALGAS) {
+    rh = d * sqrt_h3(i1);
+    errcode = eos_pressure(P, rh, en, &n.pe, &n.dprdrh, &n.dprden);
+    df = n.dprdrh * (rh * v2 * rsqrt_h3(i1) / (en + pr)) + n.dprden * v2 - 1.;
+  } else {
+    errcode = eos_pressure_it(P, 0., en, &n.pe, &n.dprdrh, &n.dprden, n.at);
+    df = fma(n.dprden, v2, -1.);
+  }
+  dpr = (pr - n.pe) * rcp_h3(df);
+#endif
+  return false;
+}
+__device__ __forceinline__ void fluid_rho(double d, double v2, double& rh) {
+#ifndef ECHO_EXACT
+  rh = d * sqrt_h3(1. - v2);
+#endif
+}
 
 // ---------------------------------------------------------------------------
 // Resistive MHD (MHD = 2): Ohm's law and the implicit E solve.
@@ -746,7 +892,7 @@ __device__ __forceinline__ void cross_contra(const Metric& M, const double* a, c
   double gp = M.gp;
   o[0] = gp * (a[1] * b[2] - a[2] * b[1]);
   o[1] = gp * (a[2] * b[0] - a[0] * b[2]);
-  o[2] = gp / M.g3 * (a[0] * b[1] - a[1] * b[0]);
+  o[2] = over_g3(M, gp) * (a[0] * b[1] - a[1] * b[0]);
 }
 
 // stiff E source before the sqrt(-g) factor (system.f90:1656-1660):
@@ -770,9 +916,13 @@ __device__ __forceinline__ void ohm_stiff(const DevPhys& P, const Metric& M, con
 // lam = h gamma sigma, mu = h gamma sigma_chi; solved by cofactors
 __device__ __forceinline__ void ohm_solve(const DevPhys& P, const Metric& M, const double* Es, const double* vel,
                                           const double* B, double h, double* E) {
-  double g3 = M.g3, gp = M.gp, gq = M.gp / M.g3;
+  double g3 = M.g3, gp = M.gp, gq = over_g3(M, M.gp);
   double v2 = vel[0] * vel[0] + vel[1] * vel[1] + g3 * (vel[2] * vel[2]);
+#ifdef ECHO_EXACT
   double glf = 1. / sqrt(1. - v2);
+#else
+  double glf = rsqrt_h3(1. - v2);
+#endif
   double lam = h * glf * P.sigma_el, mu = h * glf * P.sigma_chiral;
   double vxb[3];
   cross_contra(M, vel, B, vxb);
@@ -796,9 +946,16 @@ __device__ __forceinline__ void ohm_solve(const DevPhys& P, const Metric& M, con
   double c21 = Mx[0][2] * Mx[1][0] - Mx[0][0] * Mx[1][2];
   double c22 = Mx[0][0] * Mx[1][1] - Mx[0][1] * Mx[1][0];
   double det = Mx[0][0] * c00 + Mx[0][1] * c01 + Mx[0][2] * c02;
+#ifdef ECHO_EXACT
   E[0] = (c00 * r[0] + c10 * r[1] + c20 * r[2]) / det;
   E[1] = (c01 * r[0] + c11 * r[1] + c21 * r[2]) / det;
   E[2] = (c02 * r[0] + c12 * r[1] + c22 * r[2]) / det;
+#else
+  const double rdet = rcp_h3(det);
+  E[0] = (c00 * r[0] + c10 * r[1] + c20 * r[2]) * rdet;
+  E[1] = (c01 * r[0] + c11 * r[1] + c21 * r[2]) * rdet;
+  E[2] = (c02 * r[0] + c12 * r[1] + c22 * r[2]) * rdet;
+#endif
 }
 
 // Resistive con2prim with the implicit Ohm's law of an IMEX stage (the
@@ -855,26 +1012,16 @@ inline __device__ int cons2prim_res(const DevPhys& P, const Metric& M, double* u
     }
     double Ec[3] = {E[0], E[1], E[2] * g3}, EXB[3];
     exb(M, Ec, B[0], B[1], B[2], EXB);
-    double E2 = Ec[0] * Ec[0] + Ec[1] * Ec[1] + (Ec[2] * Ec[2]) / g3;
-    double sx = S[0] - EXB[0], sy = S[1] - EXB[1], sz = (S[2] - EXB[2]) / g3;
+    double E2 = Ec[0] * Ec[0] + Ec[1] * Ec[1] + over_g3(M, Ec[2] * Ec[2]);
+    double sx = S[0] - EXB[0], sy = S[1] - EXB[1], sz = over_g3(M, S[2] - EXB[2]);
     double et = U - 0.5 * (E2 + B2);
     double s2 = g1 * sx * sx + g2 * sy * sy + g3 * sz * sz;
-    double w = 0, v2 = 0, glf, en, drhdpr, dendpr, pr_eos = 0, dprdrh = 0, dprden = 0, f, df, dpr;
+    double w = 0, v2 = 0, dpr;
+    FluidNewton fn;
     bool newton_ok = false;
     int iter;
     for (iter = 1; iter <= 100; iter++) {
-      w = et + pr;
-      v2 = s2 / (w * w);
-      if (v2 >= 1.) break;
-      glf = 1. / sqrt(1. - v2);
-      rh = d / glf;
-      en = w * (1. - v2) - pr;
-      drhdpr = rh * v2 * glf / (en + pr);
-      dendpr = v2;
-      errcode = eos_pressure(P, rh, en, &pr_eos, &dprdrh, &dprden);
-      f = pr_eos - pr;
-      df = dprdrh * drhdpr + dprden * dendpr - 1.;
-      dpr = -f / df;
+      if (fluid_step(P, d, s2, et, 0., pr, fn, w, v2, rh, dpr, errcode)) break;
       if (fabs(dpr) < ntol * pr) {
         newton_ok = true;
         break;
@@ -887,6 +1034,7 @@ inline __device__ int cons2prim_res(const DevPhys& P, const Metric& M, double* u
       pr = pr + dpr;
     }
     total += iter;
+    if (v2 < 1.) fluid_rho(d, v2, rh);
     if (cap < 100 && (v2 >= 1. || !newton_ok)) {
       // the seed failed: the fixed point from the warm start
       if (seed_failed) *seed_failed |= 1;
@@ -904,7 +1052,12 @@ inline __device__ int cons2prim_res(const DevPhys& P, const Metric& M, double* u
     }
     const bool seeded_pass = cap < 100;  // another pass at the full tolerance follows
     cap = 1 << 30;
+#ifdef ECHO_EXACT
     double vn0 = sx / w, vn1 = sy / w, vn2 = sz / w;
+#else
+    const double rw = rcp_h3(w);
+    double vn0 = sx * rw, vn1 = sy * rw, vn2 = sz * rw;
+#endif
     double dv = fmax3(fabs(vn0 - vel[0]), fabs(vn1 - vel[1]), fabs(vn2 - vel[2]) * gp);
     vel[0] = vn0;
     vel[1] = vn1;
@@ -942,7 +1095,10 @@ __host__ __device__ __forceinline__ bool c2p_alt_algo(int algo) {
   return algo != ECHO_C2P_BRENT && algo != ECHO_C2P_NEWTON && algo != ECHO_C2P_MLP;
 }
 
-template <int KIND, bool ALT = false>
+// ALGO: the ideal-MHD solver fixed at compile time (C2P_NEWTON: Newton, with
+// BRENTM out of line for the cells it does not solve) or by `algo` (C2P_ANY).
+enum { C2P_ANY = 0, C2P_NEWTON = 1 };
+template <int KIND, bool ALT = false, int ALGO = C2P_ANY>
 __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol, const double* u,
                          double* v, int* iters, const float* seed = nullptr, int* seed_failed = nullptr,
                          double h = 0.) {
@@ -960,36 +1116,33 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
     double d = gm * u[KRH];
     double sx = gm * u[KVX];
     double sy = gm * u[KVY];
-    double sz = gm * u[KVZ] / g3;
+    double sz = over_g3(M, gm * u[KVZ]);
     double et = gm * u[KPR];
     double s2 = g1 * sx * sx + g2 * sy * sy + g3 * sz * sz;
-    double pr = v[KPR], w = 0, v2, glf, rh = 0, en, drhdpr, dendpr;
-    double pr_eos = 0, dprdrh = 0, dprden = 0, f, df, dpr;
+    double pr = v[KPR], w = 0, v2 = 0, rh = 0, dpr;
+    FluidNewton fn;
     int iter;
     for (iter = 1; iter <= 100; iter++) {
-      w = et + pr;
-      v2 = s2 / (w * w);
-      if (v2 >= 1.) {
+      if (fluid_step(P, d, s2, et, 0., pr, fn, w, v2, rh, dpr, errcode)) {
         *iters = iter;
         return 777;
       }
-      glf = 1. / sqrt(1. - v2);
-      rh = d / glf;
-      en = w * (1. - v2) - pr;
-      drhdpr = rh * v2 * glf / (en + pr);
-      dendpr = v2;
-      errcode = eos_pressure(P, rh, en, &pr_eos, &dprdrh, &dprden);
-      f = pr_eos - pr;
-      df = dprdrh * drhdpr + dprden * dendpr - 1.;
-      dpr = -f / df;
       if (fabs(dpr) < ntol * pr) break;
       pr = pr + dpr;
     }
     *iters = iter;
+    fluid_rho(d, v2, rh);
     v[KRH] = rh;
+#ifdef ECHO_EXACT
     v[KVX] = sx / w;
     v[KVY] = sy / w;
     v[KVZ] = sz / w;
+#else
+    const double rw = rcp_h3(w);
+    v[KVX] = sx * rw;
+    v[KVY] = sy * rw;
+    v[KVZ] = sz * rw;
+#endif
     v[KPR] = pr;
     if (pr <= 0) errcode = 777;
     return errcode;
@@ -1010,13 +1163,20 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
 #pragma unroll
     for (int k = 0; k < T::NV; k++) uin[k] = gm * u[k];
     double d = uin[KRH];
+#ifdef ECHO_EXACT
 #pragma unroll
     for (int k = KPIBU; k <= KPIZZ; k++) v[k] = uin[k] / uin[KRH];
+#else
+    const double rd = rcp_h3(uin[KRH]);
+#pragma unroll
+    for (int k = KPIBU; k <= KPIZZ; k++) v[k] = uin[k] * rd;
+#endif
     double vx = v[KVX], vy = v[KVY], vz = v[KVZ];
     double v2 = g1 * (vx * vx) + g2 * (vy * vy) + g3 * (vz * vz);
 #pragma unroll
     for (int k = 0; k < T::NV; k++) vprim[k] = v[k];
-    double rh = 0, pr = 0, glf, en, drhdpr, dendpr, pr_eos = 0, dprdrh = 0, dprden = 0, f, df, dpr;
+    double rh = 0, pr = 0, dpr;
+    FluidNewton fn;
     double et = gm * u[KPR];
     const bool conv = algo == ECHO_C2P_NEWTON || algo == ECHO_C2P_MLP;
     double p0 = v[KPR];  // where each pass's Newton starts
@@ -1047,23 +1207,14 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
       double sx_cov = uin[KVX] - pi.tx;
       double sy_cov = uin[KVY] - pi.ty;
       double sz_cov = uin[KVZ] - pi.tz * g3;
-      double sx = sx_cov, sy = sy_cov, sz = sz_cov / g3;
+      double sx = sx_cov, sy = sy_cov, sz = over_g3(M, sz_cov);
       double s2 = sx * sx_cov + sy * sy_cov + sz * sz_cov;
       pr = p0;
       bool newton_ok = false;
+      double wn = 0;
       for (int ip = 1; ip <= 100; ip++) {
         tot++;
-        v2 = s2 / ((en1 + pr) * (en1 + pr));
-        if (v2 >= 1.) break;
-        glf = 1. / sqrt(1. - v2);
-        rh = d / glf;
-        en = (en1 + pr) * (1. - v2) - pr - vprim[KPIBU];
-        drhdpr = rh * v2 * glf / (en + pr);
-        dendpr = v2;
-        errcode = eos_pressure(P, rh, en, &pr_eos, &dprdrh, &dprden);
-        f = pr_eos - pr;
-        df = dprdrh * drhdpr + dprden * dendpr - 1.;
-        dpr = -f / df;
+        if (fluid_step(P, d, s2, en1, vprim[KPIBU], pr, fn, wn, v2, rh, dpr, errcode)) break;
         if (fabs(dpr) < ntol * pr) {
           newton_ok = true;
           break;
@@ -1092,11 +1243,14 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
       }
       const bool seeded_pass = cap < 100;  // another pass at the full tolerance follows
       cap = 1 << 30;
-      double nvx = sx / (en1 + pr);
+#ifdef ECHO_EXACT
+      double nvx = sx / (en1 + pr), nvy = sy / (en1 + pr), nvz = sz / (en1 + pr);
+#else
+      const double rw = rcp_h3(en1 + pr);
+      double nvx = sx * rw, nvy = sy * rw, nvz = sz * rw;
+#endif
       if (fabs(nvx) < eps) nvx = 0.;
-      double nvy = sy / (en1 + pr);
       if (fabs(nvy) < eps) nvy = 0.;
-      double nvz = sz / (en1 + pr);
       if (fabs(nvz) < eps) nvz = 0.;
       // the converged passes' test: a component below eps is zeroed (above), so
       // one that sits at that threshold can alternate between 0 and just above
@@ -1119,6 +1273,7 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
       }
     }
     *iters = tot;
+    fluid_rho(d, v2, rh);
     v[KRH] = rh;
     v[KVX] = vx;
     v[KVY] = vy;
@@ -1148,7 +1303,7 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
     double B2 = bx * bx + by * by + bz * bz * g3;
     double SB = sx * bx + sy * by + sz * bz;
     double SB2 = SB * SB;
-    double SS2 = sx * sx + sy * sy + sz * sz / g3;
+    double SS2 = sx * sx + sy * sy + over_g3(M, sz * sz);
     double rh = v[KRH], vx = v[KVX], vy = v[KVY], vz = v[KVZ], pr = v[KPR];
     double en = 0;
     errcode = eos_energy(P, rh, &en, pr);
@@ -1159,7 +1314,8 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
     X[2] = pr;
     Sist3 s = {B2, SB2, SS2, UU, DD, 1.0 / (fabs(UU) + B2)};
     int nfev = 0;
-    if (algo == ECHO_C2P_NEWTON || algo == ECHO_C2P_MLP) {
+    bool brent = true;
+    if (ALGO == C2P_NEWTON || algo == ECHO_C2P_NEWTON || algo == ECHO_C2P_MLP) {
       int it = -1, used = 0;
       if (algo == ECHO_C2P_MLP && seed) {
         // learned seed: x = v^2 and p = q U, y from sist3's third equation
@@ -1189,22 +1345,32 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
           it += used;
         }
       }
-      if (it > 0) {
+      brent = it <= 0;
+      if (!brent)
         nfev = it;
-      } else {
+      else if (seed_failed)
+        *seed_failed |= 2;  // a bracketed fallback, counted on its own
+    }
+    if (brent) {
+      if (ALGO == C2P_NEWTON)
+        (void)brentm3_call(P, s, X, &nfev);
+      else
         (void)brentm3(P, s, X, 1.e-14, 1.e-14, 300, 3, &nfev);
-        if (seed_failed) *seed_failed |= 2;  // a bracketed fallback, counted on its own
-      }
-    } else {
-      (void)brentm3(P, s, X, 1.e-14, 1.e-14, 300, 3, &nfev);
     }
     *iters = nfev;
     double xs = X[0], ys = X[1];
     pr = X[2];
     rh = DD * sqrt(1 - xs);
+#ifdef ECHO_EXACT
     vx = (sx + SB * bx / ys) / (ys + B2);
     vy = (sy + SB * by / ys) / (ys + B2);
     vz = (sz / g3 + SB * bz / ys) / (ys + B2);
+#else
+    const double rb = rcp_h3(ys + B2), q = SB * rcp_h3(ys);
+    vx = (sx + q * bx) * rb;
+    vy = (sy + q * by) * rb;
+    vz = (over_g3(M, sz) + q * bz) * rb;
+#endif
     v[KRH] = rh;
     v[KVX] = vx;
     v[KVY] = vy;
@@ -1276,6 +1442,88 @@ __device__ __forceinline__ void get_sigma(const DevPhys& P, const Metric& M, con
   }
 }
 
+#ifndef ECHO_EXACT
+// Product build, Milne coordinates: the Israel-Stewart sources below (before
+// the factor sqrt(-g)) in covariant form.  sigma^ij = (nabla^i u^j + nabla^j u^i
+// + u^i a^j + u^j a^i) / 2 - Delta^ij theta / 3 with the Christoffel terms
+// Gamma^t_ee = tau, Gamma^e_te = 1 / tau in the velocity gradient is get_sigma's
+// expression term by term; the gradients along the flow (sum_der_*) are its
+// a^i without them.  About 250 FP64 operations and one division by tau, where
+// the expanded form divides by tau some forty times.
+template <int KIND>
+__device__ __forceinline__ int visc_source_milne(const DevPhys& P, const Metric& M, double* v, const double* d,
+                                                 double en, const EosAt& at, double glf, double* src,
+                                                 double* kap) {
+  const double g3 = M.g3, t = M.t, it = M.gm, ig3 = M.ig3;
+  double eta, zeta = 0., itau;  // 1 / tau_pi (tau_Pi is the same)
+  if (at.h) {
+    // get_viscous_parameters in the interval of e(p): T beside it in the table
+    const double h = en + v[KPR], t1 = __ldg(P.tT + at.h - 2), t2 = __ldg(P.tT + at.h - 1);
+    const double temp = fma(t2 - t1, (v[KPR] - at.p0) * rcp_h3(at.hi - at.p0), t1);
+    if (en < P.emin) return 131;
+    if (en > P.emax) return 132;
+    eta = P.init_type == 2 ? P.eta_over_s : 0.197326 * P.eta_over_s * (h * rcp_h3(temp));
+    if (P.bulkvis) zeta = 2. * eta * (1. / 3. - eos_sound_at(P, at, en));
+    itau = h * rcp_h3((P.init_type == 5 ? 5. : P.tau_pi_coeff) * eta);
+  } else {
+    double tau_pi, tau_pi_big;
+    const int err = viscous_parameters(P, v[KRH], v[KPR], &eta, &zeta, &tau_pi, &tau_pi_big);
+    if (err) return err;
+    itau = 1. / tau_pi;
+  }
+  Pit pi;
+  derived_pi_any(P, M, v, pi);
+  const double vx = v[KVX], vy = v[KVY], vz = v[KVZ], pr = v[KPR], bu = v[KPIBU];
+  const double ux = glf * vx, uy = glf * vy, uz = glf * vz;
+  // u^n d_n u^m
+  const double ft = glf * d[DTT] + ux * d[DTX] + uy * d[DTY] + uz * d[DTZ];
+  const double fx = glf * d[DXT] + ux * d[DXX] + uy * d[DXY] + uz * d[DXZ];
+  const double fy = glf * d[DYT] + ux * d[DYX] + uy * d[DYY] + uz * d[DYZ];
+  const double fz = glf * d[DZT] + ux * d[DZX] + uy * d[DZY] + uz * d[DZZ];
+  const double theta = d[DTT] + d[DXX] + d[DYY] + d[DZZ] + glf * it, th3 = theta * (1. / 3.);
+  const double az = fz + 2. * glf * it * uz;  // a^eta
+  const double w = (en + pr + bu) * (glf * glf);
+  src[KPR] = -t * (w * (vz * vz) + (pr + bu) * ig3 + v[KPIZZ]);
+  const double dil = (4. / 3.) * theta + itau, rh = v[KRH];
+  src[KPIBU] = -rh * (bu * dil + zeta * theta * itau);
+  // the covariant gradients along the flow as the relaxation equations take them
+  const double lt = -ft, lx = fx, ly = fy, lz = g3 * fz + 2. * t * uz;
+  const double xx = v[KPIXX], yy = v[KPIYY], zz = v[KPIZZ], xy = v[KPIXY], xz = v[KPIXZ], yz = v[KPIYZ];
+  const double rx = pi.tx * lt + xx * lx + xy * ly + xz * lz;
+  const double ry = pi.ty * lt + xy * lx + yy * ly + yz * lz;
+  const double rz = pi.tz * lt + xz * lx + yz * ly + zz * lz;
+  const double et = 2. * eta * itau;
+  {
+    const double s = d[DXX] + ux * fx - (1. + ux * ux) * th3;
+    src[KPIXX] = rh * (2. * ux * rx - xx * dil - et * s);
+  }
+  {
+    const double s = d[DYY] + uy * fy - (1. + uy * uy) * th3;
+    src[KPIYY] = rh * (2. * uy * ry - yy * dil - et * s);
+  }
+  {
+    const double s = 0.5 * (d[DXY] + d[DYX] + uy * fx + ux * fy) - ux * uy * th3;
+    src[KPIXY] = rh * (uy * rx + ux * ry - xy * dil - et * s);
+  }
+  {
+    const double s = (d[DZZ] + glf * it) * ig3 + uz * az - (ig3 + uz * uz) * th3;
+    src[KPIZZ] = rh * (2. * uz * rz - zz * dil - et * s - 2. * it * (glf * zz + uz * pi.tz));
+  }
+  {
+    const double s = 0.5 * (ig3 * d[DXZ] + d[DZX] + uz * fx + ux * az) - ux * uz * th3;
+    src[KPIXZ] = rh * (uz * rx + ux * rz - xz * dil - et * s - it * (glf * xz + uz * pi.tx));
+  }
+  {
+    const double s = 0.5 * (ig3 * d[DYZ] + d[DZY] + uz * fy + uy * az) - uy * uz * th3;
+    src[KPIYZ] = rh * (uz * ry + uy * rz - yz * dil - et * s - it * (glf * yz + uz * pi.ty));
+  }
+  if (kap) {
+    kap[0] = kap[1] = itau * rcp_h3(glf);
+  }
+  return 0;
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // system_source (system.f90:1587-1842) without the resistive terms.
 // v: primitives of the cell (modified copy), dv: its 16 derivatives.
@@ -1294,10 +1542,19 @@ __device__ int system_source(const DevPhys& P, const Metric& M, double* v, const
   for (int k = 0; k < T::NV; k++) src[k] = 0.;
   double rh = v[KRH], vx = v[KVX], vy = v[KVY], vz = v[KVZ], pr = v[KPR];
   double en = 0;
+#ifdef ECHO_EXACT
   int err = eos_energy(P, rh, &en, pr);
+#else
+  EosAt at;
+  int err = eos_energy_h(P, rh, &en, pr, at);
+#endif
   if (err) return err;
   double v2 = g1 * vx * vx + g2 * vy * vy + g3 * vz * vz;
+#ifdef ECHO_EXACT
   double glf = 1. / sqrt(1. - v2);
+#else
+  double glf = rsqrt_h3(1. - v2);
+#endif
   double ut = glf;
   const double lambda0 = 1., lambda1 = 1., lambda2 = 0.;
   if (!T::VISC) {
@@ -1310,14 +1567,19 @@ __device__ int system_source(const DevPhys& P, const Metric& M, double* v, const
                                  // resistive runs (system.f90:1641)
         double bx = v[KBX], by = v[KBY], bz = v[KBZ];
         double B2 = bx * bx + by * by + (bz * bz) * g3;
-        double E2 = E[0] * E[0] + E[1] * E[1] + (E[2] * E[2]) / g3;
+        double E2 = E[0] * E[0] + E[1] * E[1] + over_g3(M, E[2] * E[2]);
         double EEM = 0.5 * (E2 + B2);
-        double e3g = E[2] / g3;
-        src[KPR] = -t * (ww * vz * vz - e3g * e3g - bz * bz + (EEM + pr) / g3);
+        double e3g = over_g3(M, E[2]);
+        src[KPR] = -t * (ww * vz * vz - e3g * e3g - bz * bz + over_g3(M, EEM + pr));
       } else {
-        src[KPR] = -t * (ww * vz * vz + pr / g3);
+        src[KPR] = -t * (ww * vz * vz + over_g3(M, pr));
       }
     }
+#ifndef ECHO_EXACT
+  } else if (P.coordinates == ECHO_BJORKEN) {
+    err = visc_source_milne<KIND>(P, M, v, dv, en, at, glf, src, kap);
+    if (err) return err;
+#endif
   } else {
     double sigma[6], eta, zeta, tau_pi, tau_pi_big;
     enum { SXX = 0, SYY = 1, SZZ = 2, SXY = 3, SXZ = 4, SYZ = 5 };

@@ -86,22 +86,55 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
                     int** d_bk) {
   *d_tab = nullptr;
   int nt = 0;
+  size_t ncol = 0;  // doubles of the columns, a whole number of 64-byte lines
+  std::vector<int> be, bp;
+  long long ke0 = 0, kp0 = 0;
+  bool fast = false;  // e and p strictly increasing: the O(1) bracket search
   if (eos_table && n_eos > 0) {
-    // columns T, e, p, c_s^2, then the interval slopes de/dp, d(c_s^2)/de
-    // and dp/de = (dp/dT)/(de/dT) (get_pressure's derivative, eos.f90:458-462)
     nt = n_eos;
-    std::vector<double> cols((size_t)7 * n_eos, 0.0);
-    for (int i = 0; i < n_eos; i++)
-      for (int q = 0; q < 4; q++) cols[(size_t)q * n_eos + i] = eos_table[4 * i + q];
-    for (int i = 0; i + 1 < n_eos; i++) {
-      const double* a = eos_table + 4 * i;
-      const double* b = a + 4;
-      cols[(size_t)4 * n_eos + i] = (b[1] - a[1]) / (b[2] - a[2]);
-      cols[(size_t)5 * n_eos + i] = (b[3] - a[3]) / (b[1] - a[1]);
-      cols[(size_t)6 * n_eos + i] = ((b[2] - a[2]) / (b[0] - a[0])) / ((b[1] - a[1]) / (b[0] - a[0]));
+    std::vector<double> te(nt), tp(nt);
+    for (int i = 0; i < nt; i++) {
+      te[i] = eos_table[4 * i + 1];
+      tp[i] = eos_table[4 * i + 2];
     }
-    CK(cudaMalloc(d_tab, sizeof(double) * 7 * n_eos));
-    CK(cudaMemcpy(*d_tab, cols.data(), sizeof(double) * 7 * n_eos, cudaMemcpyHostToDevice));
+    fast = echo_make_buckets(te.data(), nt, be, ke0) && echo_make_buckets(tp.data(), nt, bp, kp0);
+    // columns T, e, p, c_s^2; product build: the interval records and the
+    // buckets of e and p after them
+    ncol = ((size_t)4 * nt + 7) / 8 * 8;
+    std::vector<double> cols(ncol, 0.0);
+    for (int i = 0; i < nt; i++)
+      for (int q = 0; q < 4; q++) cols[(size_t)q * nt + i] = eos_table[4 * i + q];
+#ifndef ECHO_EXACT
+    if (fast) {
+      std::vector<EosRec> rec(nt);
+      memset(rec.data(), 0, sizeof(EosRec) * nt);
+      for (int i = 0; i + 1 < nt; i++) {
+        const double* a = eos_table + 4 * i;
+        const double* b = a + 4;
+        rec[i].tp = a[2];
+        rec[i].te = a[1];
+        rec[i].tp1 = b[2];
+        rec[i].te1 = b[1];
+        rec[i].tc = a[3];
+        rec[i].sl_ep = (b[1] - a[1]) / (b[2] - a[2]);
+        rec[i].sl_ce = (b[3] - a[3]) / (b[1] - a[1]);
+        rec[i].sl_pe = ((b[2] - a[2]) / (b[0] - a[0])) / ((b[1] - a[1]) / (b[0] - a[0]));  // eos.f90:458-462
+      }
+      std::vector<EosBucket> q(be.size() + bp.size());
+      for (size_t i = 0; i < q.size(); i++) {
+        const bool e = i < be.size();
+        q[i].h = e ? be[i] : bp[i - be.size()];
+        q[i].node = (e ? te : tp)[q[i].h - 1];
+        q[i].pad = 0;
+      }
+      const size_t nrec = sizeof(EosRec) / sizeof(double) * nt, nq = sizeof(EosBucket) / sizeof(double) * q.size();
+      cols.resize(ncol + nrec + nq);
+      memcpy(cols.data() + ncol, rec.data(), sizeof(double) * nrec);
+      memcpy(cols.data() + ncol + nrec, q.data(), sizeof(double) * nq);
+    }
+#endif
+    CK(cudaMalloc(d_tab, sizeof(double) * cols.size()));
+    CK(cudaMemcpy(*d_tab, cols.data(), sizeof(double) * cols.size(), cudaMemcpyHostToDevice));
   }
   P->eqstate = p->eqstate;
   P->coordinates = p->coordinates;
@@ -123,31 +156,30 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
   P->sigma_el = p->sigma_el;
   P->sigma_chiral = p->sigma_chiral;
   P->bke = P->bkp = nullptr;
-  P->sl_ep = P->sl_ce = P->sl_pe = nullptr;
+  P->rec = nullptr;
+  P->qe = P->qp = nullptr;
+  P->emin = P->emax = P->pmin = P->pmax = 0.;
   *d_bk = nullptr;
-  if (nt > 0) {
-    std::vector<double> te(nt), tp(nt);
-    for (int i = 0; i < nt; i++) {
-      te[i] = eos_table[4 * i + 1];
-      tp[i] = eos_table[4 * i + 2];
-    }
-    std::vector<int> be, bp;
-    long long ke0 = 0, kp0 = 0;
-    if (echo_make_buckets(te.data(), nt, be, ke0) && echo_make_buckets(tp.data(), nt, bp, kp0)) {
-      CK(cudaMalloc(d_bk, sizeof(int) * (be.size() + bp.size())));
-      CK(cudaMemcpy(*d_bk, be.data(), sizeof(int) * be.size(), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(*d_bk + be.size(), bp.data(), sizeof(int) * bp.size(), cudaMemcpyHostToDevice));
-      P->bke = *d_bk;
-      P->bkp = *d_bk + be.size();
-      P->bke0 = ke0;
-      P->bkp0 = kp0;
-      P->nbke = (int)be.size();
-      P->nbkp = (int)bp.size();
-      // strictly increasing e and p: every interval has a finite slope
-      P->sl_ep = *d_tab + 4 * nt;
-      P->sl_ce = *d_tab + 5 * nt;
-      P->sl_pe = *d_tab + 6 * nt;
-    }
+  if (fast) {
+    P->bke0 = ke0;
+    P->bkp0 = kp0;
+    P->nbke = (int)be.size();
+    P->nbkp = (int)bp.size();
+#ifdef ECHO_EXACT
+    CK(cudaMalloc(d_bk, sizeof(int) * (be.size() + bp.size())));
+    CK(cudaMemcpy(*d_bk, be.data(), sizeof(int) * be.size(), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(*d_bk + be.size(), bp.data(), sizeof(int) * bp.size(), cudaMemcpyHostToDevice));
+    P->bke = *d_bk;
+    P->bkp = *d_bk + be.size();
+#else
+    P->rec = (const EosRec*)(*d_tab + ncol);
+    P->qe = (const EosBucket*)(P->rec + nt);
+    P->qp = P->qe + be.size();
+    P->emin = eos_table[1];
+    P->emax = eos_table[4 * (size_t)(nt - 1) + 1];
+    P->pmin = eos_table[2];
+    P->pmax = eos_table[4 * (size_t)(nt - 1) + 2];
+#endif
   }
   return ECHO_OK;
 }

@@ -1,33 +1,35 @@
 // faces.cuh -- the flux sweeps of a stage, cell-centred tiles.
 //
-// A block owns a tile of C = 2^lc consecutive cells (ghost cells included) and
+// A block owns a tile of C = 2^LC consecutive cells (ghost cells included) and
 // the faces between them.  Phase 1: every thread reconstructs both face states
-// of its cell, one variable after another (recon_cell), into shared memory.
-// Phase 2: one thread per face takes the upper state of the cell below and the
-// lower state of the cell above and computes the HLL flux.
+// of its CPT neighbouring cells, one variable after another (recon_cells), into
+// shared memory.  Phase 2: the flux of a face takes the upper state of the cell
+// below and the lower state of the cell above.
 //
-// What bounds it: FP64 issue.  One thread per face with all its variables in
-// registers (the arrangement before) evaluated the smoothness indicators of a
-// cell twice, unrolled every variable into one body and spilled about 600 bytes
-// a thread at the 72 registers its occupancy needed.  Here a cell's indicators
-// serve both its faces, the reconstruction is a rolled loop over the variables
-// (one variable's operands live, the next one's loads in flight) and the flux
+// What bounds it: L1 and FP64 issue, in phases that the blocks of an SM overlap.
+// One thread per face with all its variables in registers (the arrangement
+// before) evaluated the smoothness indicators of a cell twice, unrolled every
+// variable into one body and spilled about 600 bytes a thread at the 72
+// registers its occupancy needed.  Here a cell's indicators serve both its
+// faces, two neighbouring cells of a thread share loads (6 for 10) and
+// differences, the reconstruction is a loop over the variables and the flux
 // reads its operands from shared memory where it uses them.
 //
-// Tiles.  Along x the cells 0..nx+1 of all pencils are numbered through and
-// tile t covers C of them from t (C - 1) on, so that C - 1 faces (2 % of them
-// between two pencils) come from C cells.  Along y and eta a tile is W = 2^lw
-// neighbouring pencils (consecutive in memory) by C / W cells, one row more
-// than it has faces; W = 16 keeps every load at whole 128-byte lines.
+// Tiles.  Along x the cells 0..nx+1 of all pencils (padded to an even number)
+// are numbered through and tile t covers C of them from t (C - 2) on.  Along y
+// and eta a tile is W = 2^lw neighbouring pencils (consecutive in memory) by
+// C / W cells, one row more than it has faces; W = 16 keeps every load at whole
+// 128-byte lines.
 //
-// Measured (97 x 97 x 81 ideal RMHD, B200): x / y / eta sweep 111 / 108 / 114 us
-// with one thread per face, 80 / 82 / 86 us here, 39 to 44 million warp
-// instructions instead of 60 to 64 (half of them FP64 in both); resistive
-// 193 x 193 x 129: 742 / 733 / 844 us before, 476 / 527 / 549 us here.
+// Measured, x / y / eta us a launch, one thread per face before and this: ideal
+// RMHD 97 x 97 x 81 111 / 108 / 114 and 76 / 70 / 73; resistive 193 x 193 x 129
+// 742 / 733 / 844 and 451 / 498 / 520.  With the loads, the reconstruction or
+// the flux left out in turn the RMHD x sweep took 62, 69 and 72 us: no one of
+// them bounds it.
 #pragma once
 
 #ifndef ECHO_SWEEP_UNROLL
-#define ECHO_SWEEP_UNROLL 3
+#define ECHO_SWEEP_UNROLL 2
 #endif
 
 namespace echo {
@@ -35,7 +37,7 @@ namespace echo {
 struct SweepArgs {
   FaceArgs A[3];          // x, y, eta
   unsigned first[4];      // block range of each direction
-  int lw;                 // log2 of the pencils of a tile (y, eta)
+  int lw;                 // log2 of the pencils of a y or eta tile
 };
 
 // 64 KB of shared memory a block at most: 2 x (NV + 4) x 256 doubles
@@ -53,8 +55,8 @@ __host__ __device__ constexpr size_t tile_smem(int lc) {
 __host__ __device__ inline unsigned tiles_of(const Grid& g, int dir, int lc, int lw) {
   const unsigned C = 1u << lc;
   if (dir == 0) {
-    const unsigned e = (unsigned)(g.nx + 2) * (unsigned)g.ny * (unsigned)g.nz - 1;  // pairs of neighbours
-    return (e + C - 2) / (C - 1);
+    const unsigned e = (((unsigned)g.nx + 3u) & ~1u) * (unsigned)g.ny * (unsigned)g.nz;
+    return (e + C - 3) / (C - 2);
   }
   const unsigned n = (unsigned)(dir == 1 ? g.ny : g.nz), cols = (unsigned)g.nx * (unsigned)(dir == 1 ? g.nz : g.ny);
   const unsigned rows = (C >> lw) - 1;
@@ -65,11 +67,10 @@ __host__ __device__ inline unsigned tiles_of(const Grid& g, int dir, int lc, int
 // What the flux of one side of a face needs beside the primitives w[k * ld].
 struct FaceSide {
   double ww, D, em;  // w gamma^2, rho gamma, electromagnetic energy
+  double i1, vB;     // ideal MHD: 1 / gamma^2 and v.B, with ww = w gamma^2 + B^2 and em = b^2 / 2
 };
 
 // Energy density, enthalpy and the signal speeds of one side (system_flux).
-// With w = e + p, b = B^2 - E^2 and a^2 = (c_s^2 w + b) / (w + b), the fast
-// speeds' 1 / (1 - v^2 a^2) and 1 / (w + b) are one reciprocal.
 template <int KIND, int DIR>
 __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, const double* w, int ld, FaceSide& s,
                                            double& vfp, double& vfm) {
@@ -77,8 +78,8 @@ __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, co
   const double rh = w[KRH * ld], pr = w[KPR * ld];
   const double vx = w[KVX * ld], vy = w[KVY * ld], vz = w[KVZ * ld];
   double en = 0.;
-  int hb = 0;
-  int err = eos_energy_h(P, rh, &en, pr, &hb);
+  EosAt at;
+  int err = eos_energy_h(P, rh, &en, pr, at);
   if (err) return err;
   const double v2 = vx * vx + vy * vy + M.g3 * (vz * vz);
   if (v2 > 1) return 333;
@@ -86,21 +87,20 @@ __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, co
   s.ww = (T::VISC ? h + w[KPIBU * ld] : h) * (glf * glf);
   s.D = rh * glf;
   s.em = 0.;
-  double b = 0.;
+  double b = 0.;  // B^2 - E^2
   if (T::MHD) {
     const double bx = w[KBX * ld], by = w[KBY * ld], bz = w[KBZ * ld];
-    double E[3];
-    if (T::RES) {
-      E[0] = w[KEX * ld];
-      E[1] = w[KEY * ld];
-      E[2] = w[KEZ * ld] * M.g3;
-    } else {
-      e_ideal(M, vx, vy, vz, bx, by, bz, E);
-    }
-    const double E2 = E[0] * E[0] + E[1] * E[1] + M.ig3 * (E[2] * E[2]);
     const double B2 = bx * bx + by * by + M.g3 * (bz * bz);
-    s.em = 0.5 * (E2 + B2);
-    b = B2 - E2;
+    if (T::RES) {
+      const double ex = w[KEX * ld], ey = w[KEY * ld], ez = w[KEZ * ld];
+      s.em = 0.5 * (ex * ex + ey * ey + M.g3 * (ez * ez) + B2);
+    } else {
+      s.vB = vx * bx + vy * by + M.g3 * (vz * bz);
+      s.i1 = i1;
+      b = fma(s.vB, s.vB, B2 * i1);
+      s.em = 0.5 * b;
+      s.ww += B2;
+    }
   }
   if (T::RES) {
     // the light cone bounds the Riemann fan of the E, B waves
@@ -109,108 +109,156 @@ __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, co
     return 0;
   }
   double cs2 = 0.;
-  if (hb)
-    cs2 = eos_sound_at(P, hb, en);
+  if (at.h)
+    cs2 = eos_sound_at(P, at, en);
   else
     err = eos_sound(P, rh, en, pr, &cs2);
   if (err) return err;
   const double vd = DIR == 1 ? vx : DIR == 2 ? vy : vz;
-  // a^2 = N / q, 1 - a^2 = O / q, 1 - v^2 a^2 = Dn / q
-  const double q = T::MHD ? h + b : 1., N = T::MHD ? fma(cs2, h, b) : cs2, O = T::MHD ? h - cs2 * h : 1. - cs2;
-  const double Dn = fma(-v2, N, q), r = rcp_h3(Dn);
-  const double hd = DIR == 3 ? M.ig3 * Dn : Dn;
-  const double vf1 = O * vd * r;
-  const double vf2 = r * sqrt_h3(N * i1 * fma(-O, vd * vd, hd));
+  // in the reference's order, each operation rounded as there or within an ulp:
+  // where fluid and field are at rest the flux is (a+ f_l + a- f_r) / (a+ + a-)
+  // of equal terms, and the last bits of the speeds are its noise
+  double a2 = cs2;
+  if (T::MHD) {
+    const double ca2 = div_h3(b, b + h);
+    a2 = cs2 + ca2 - cs2 * ca2;
+  }
+  const double x = 1. - v2 * a2, den = div_h3(1., x), hd = DIR == 3 ? over_g3(M, x) : x;
+  const double vf1 = den * (1. - a2) * vd;
+  const double vf2 = den * sqrt_h3(a2 * i1 * (hd - (1. - a2) * (vd * vd)));
   vfp = vf1 + vf2;
   vfm = vf1 - vf2;
   return 0;
 }
 
-// F += c (f + lam u) of one side, f and u those of system_flux without their
-// sqrt(-g) (in c): c = a+ / (a+ + a-), lam = a- on the left,
-// c = a- / (a+ + a-), lam = -a+ on the right.
+// F += c (f + lam u) of one side for every variable but the momentum normal to
+// the face, f and u those of system_flux without their sqrt(-g) (in c): c = g
+// a+ / (a+ + a-), lam = a- on the left, c = g a- / (a+ + a-), lam = -a+ on the
+// right.  fn, un: the normal momentum's flux and value (hll_flux).
 template <int KIND, int DIR>
 __device__ __forceinline__ void side_flux(const DevPhys& P, const Metric& M, const double* w, int ld,
-                                          const FaceSide& s, double c, double lam, double* F) {
+                                          const FaceSide& s, double c, double lam, double* F, double& fn, double& un) {
   typedef Traits<KIND> T;
+  constexpr int d = DIR - 1, ia = DIR % 3, ib = (DIR + 1) % 3;
   const double v[3] = {w[KVX * ld], w[KVY * ld], w[KVZ * ld]};
-  const double pr = w[KPR * ld], g3 = M.g3;
-  const double a = v[DIR - 1] + lam;
-  F[KRH] = fma(c * s.D, a, F[KRH]);
-  const double cwa = c * s.ww * a;
-  F[KVX] = fma(cwa, v[0], F[KVX]);
-  F[KVY] = fma(cwa, v[1], F[KVY]);
-  F[KVZ] = fma(cwa, v[2] * g3, F[KVZ]);
-  double pt = pr, fe = -lam * pr;  // f + lam u beyond the w gamma^2 terms: normal stress, energy
+  const double pr = w[KPR * ld], g3 = M.g3, gd = DIR == 3 ? g3 : 1.;
+  const double a = v[d] + lam, ca = c * a;
+  F[KRH] = fma(ca, s.D, F[KRH]);
+  if (T::MHD && !T::RES) {
+    // Ideal MHD with b the field in the fluid frame: S_i = W v_i - (v.B) B_i,
+    // W = w gamma^2 + B^2; T^d_i = S_i v^d - B^d (B_i / gamma^2 + (v.B) v_i) +
+    // delta p_t, p_t = p + b^2 / 2; U = W - p_t; and v^d B^a - v^a B^d.  The
+    // same tensor as with E = -v x B, in half the operations.
+    const double B[3] = {w[KBX * ld], w[KBY * ld], w[KBZ * ld]};
+    const double cB = -c * B[d], pt = pr + s.em;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double S = fma(s.ww, v[i], -s.vB * B[i]), m = fma(s.i1, B[i], s.vB * v[i]);
+      if (i == d) {
+        un = gd * S;
+        fn = fma(gd, S * v[d] - B[d] * m, pt);
+        F[KPR] = fma(c, fma(lam, s.ww - pt, S), F[KPR]);
+      } else {
+        const double x = fma(ca, S, cB * m);
+        F[KVX + i] = i == 2 ? fma(g3, x, F[KVX + i]) : F[KVX + i] + x;
+      }
+    }
+    F[KBX + ia] = fma(ca, B[ia], fma(cB, v[ia], F[KBX + ia]));
+    F[KBX + ib] = fma(ca, B[ib], fma(cB, v[ib], F[KBX + ib]));
+    if (T::GLM) {
+      const double psi = w[T::KG * ld];
+      F[KBX + d] = fma(c, fma(lam, B[d], DIR == 3 ? over_g3(M, psi) : psi), F[KBX + d]);
+      F[T::KG] = fma(c, over_gp(M, fma(lam, psi, B[d])), F[T::KG]);
+    } else {
+      F[KBX + d] = fma(c, lam * B[d], F[KBX + d]);
+    }
+    return;
+  }
+  const double cwa = ca * s.ww, wd = s.ww * v[d];
+  // beyond the w gamma^2 v_i terms: value and flux of the momenta, energy
+  double u[3] = {0., 0., 0.}, f[3] = {0., 0., 0.}, pt = pr, fe = -lam * pr;
   if (T::VISC) {
     double p[T::NV];
 #pragma unroll
     for (int k = KVX; k < T::NV; k++) p[k] = w[k * ld];
     Pit pi;
     derived_pi_any(P, M, p, pi);  // with obtained_zz also p[KPIZZ]
-    const double pd[3] = {DIR == 1 ? p[KPIXX] : DIR == 2 ? p[KPIXY] : p[KPIXZ],
-                          DIR == 1 ? p[KPIXY] : DIR == 2 ? p[KPIYY] : p[KPIYZ],
-                          DIR == 1 ? p[KPIXZ] : DIR == 2 ? p[KPIYZ] : p[KPIZZ]};
-    F[KVX] = fma(c, fma(lam, pi.tx, pd[0]), F[KVX]);
-    F[KVY] = fma(c, fma(lam, pi.ty, pd[1]), F[KVY]);
-    F[KVZ] = fma(c * g3, fma(lam, pi.tz, pd[2]), F[KVZ]);
+    u[0] = pi.tx;
+    u[1] = pi.ty;
+    u[2] = pi.tz * g3;
+    f[0] = DIR == 1 ? p[KPIXX] : DIR == 2 ? p[KPIXY] : p[KPIXZ];
+    f[1] = DIR == 1 ? p[KPIXY] : DIR == 2 ? p[KPIYY] : p[KPIYZ];
+    f[2] = g3 * (DIR == 1 ? p[KPIXZ] : DIR == 2 ? p[KPIYZ] : p[KPIZZ]);
     pt += p[KPIBU];
     fe = fma(lam, pi.tt - pt, DIR == 1 ? pi.tx : DIR == 2 ? pi.ty : pi.tz);
-    const double cda = c * s.D * a;
+    const double cda = ca * s.D;
 #pragma unroll
     for (int k = KPIBU; k < T::NV; k++) F[k] = fma(cda, p[k], F[k]);
   }
-  if (T::MHD) {
+  if (T::RES) {
     const double B[3] = {w[KBX * ld], w[KBY * ld], w[KBZ * ld]};
-    double E[3], X[3];
-    if (T::RES) {
-      E[0] = w[KEX * ld];
-      E[1] = w[KEY * ld];
-      E[2] = w[KEZ * ld] * g3;
-    } else {
-      e_ideal(M, v[0], v[1], v[2], B[0], B[1], B[2], E);
-    }
-    exb(M, E, B[0], B[1], B[2], X);
+    const double E[3] = {w[KEX * ld], w[KEY * ld], w[KEZ * ld] * g3};
+    exb(M, E, B[0], B[1], B[2], u);
+    const double Ed = w[(KEX + d) * ld], Bd = B[d];
+#pragma unroll
+    for (int i = 0; i < 3; i++) f[i] = -Ed * E[i] - Bd * B[i] * (i == 2 ? g3 : 1.);
     pt += s.em;
-    fe = lam * (s.em - pr);
-    const double Ed = DIR == 3 ? over_g3(M, E[2]) : E[DIR - 1], Bd = B[DIR - 1];
-    F[KVX] = fma(c, lam * X[0] - Ed * E[0] - Bd * B[0], F[KVX]);
-    F[KVY] = fma(c, lam * X[1] - Ed * E[1] - Bd * B[1], F[KVY]);
-    F[KVZ] = fma(c, lam * X[2] - Ed * E[2] - Bd * (B[2] * g3), F[KVZ]);
-    fe += DIR == 3 ? over_g3(M, X[2]) : X[DIR - 1];
-    // Faraday's law: f_a = -E_b / sqrt(-g), f_b = E_a / sqrt(-g), (d, a, b) cyclic
-    const int ia = DIR % 3, ib = (DIR + 1) % 3;
+    fe = fma(lam, s.em - pr, DIR == 3 ? over_g3(M, u[d]) : u[d]);
+    // Faraday's and Ampere's laws (system.f90:1450-1452, 1491-1493,
+    // 1532-1534): f_a = -E_b / sqrt(-g), f_b = E_a / sqrt(-g) for B and
+    // B_b / sqrt(-g), -B_a / sqrt(-g) for E, (d, a, b) cyclic
     F[KBX + ia] = fma(c, fma(lam, B[ia], -E[ib] * M.gm), F[KBX + ia]);
     F[KBX + ib] = fma(c, fma(lam, B[ib], E[ia] * M.gm), F[KBX + ib]);
-    if (T::GLM) {
-      const double psi = w[T::KG * ld];
-      F[KBX + DIR - 1] = fma(c, fma(lam, Bd, DIR == 3 ? over_g3(M, psi) : psi), F[KBX + DIR - 1]);
-      F[T::KG] = fma(c, over_gp(M, fma(lam, psi, Bd)), F[T::KG]);
-    } else {
-      F[KBX + DIR - 1] = fma(c, lam * Bd, F[KBX + DIR - 1]);
-    }
-    if (T::RES) {  // Ampere's law (system.f90:1450-1452, 1491-1493, 1532-1534)
-      const double ga = ia == 2 ? g3 : 1., gb = ib == 2 ? g3 : 1.;
-      F[KEX + ia] = fma(c, fma(lam, w[(KEX + ia) * ld], B[ib] * gb * M.gm), F[KEX + ia]);
-      F[KEX + ib] = fma(c, fma(lam, w[(KEX + ib) * ld], -B[ia] * ga * M.gm), F[KEX + ib]);
-      F[KEX + DIR - 1] = fma(c, lam * w[(KEX + DIR - 1) * ld], F[KEX + DIR - 1]);
-    }
+    const double psi = w[T::KG * ld];
+    F[KBX + d] = fma(c, fma(lam, Bd, DIR == 3 ? over_g3(M, psi) : psi), F[KBX + d]);
+    F[T::KG] = fma(c, over_gp(M, fma(lam, psi, Bd)), F[T::KG]);
+    const double ga = ia == 2 ? g3 : 1., gb = ib == 2 ? g3 : 1.;
+    F[KEX + ia] = fma(c, fma(lam, w[(KEX + ia) * ld], B[ib] * gb * M.gm), F[KEX + ia]);
+    F[KEX + ib] = fma(c, fma(lam, w[(KEX + ib) * ld], -B[ia] * ga * M.gm), F[KEX + ib]);
+    F[KEX + d] = fma(c, lam * Ed, F[KEX + d]);
   }
-  F[KVX + DIR - 1] = fma(c, pt, F[KVX + DIR - 1]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    if (i == d) continue;
+    const double vi = i == 2 ? v[i] * g3 : v[i];
+    F[KVX + i] = T::VISC || T::RES ? fma(cwa, vi, fma(c, fma(lam, u[i], f[i]), F[KVX + i])) : fma(cwa, vi, F[KVX + i]);
+  }
+  un = fma(gd, wd, u[d]);
+  fn = fma(gd * wd, v[d], f[d]) + pt;
   F[KPR] += fma(c, fe, cwa);
+}
+
+// The HLL flux of a face (times sqrt(-g)) from both sides' states and signal
+// speeds ap, am (work.f90:195-229).  The momentum normal to the face holds the
+// pressure, large and nearly equal on the two sides, and its rounding is the
+// noise of the velocities: it is combined once, from both sides' whole terms.
+template <int KIND, int DIR>
+__device__ __forceinline__ void hll_flux(const DevPhys& P, const Metric& M, const double* wl, const double* wr, int ld,
+                                         const FaceSide& L, const FaceSide& R, double ap, double am, double* F) {
+  double a1 = 1.;
+  if (!(ap == 0. && am == 0.)) {
+    a1 = div_h3(1., ap + am);
+  }
+#pragma unroll
+  for (int k = 0; k < Traits<KIND>::NV; k++) F[k] = 0.;
+  const double ga = M.gp * a1;
+  double fl, ul, fr, ur;
+  side_flux<KIND, DIR>(P, M, wl, ld, L, ga * ap, am, F, fl, ul);
+  side_flux<KIND, DIR>(P, M, wr, ld, R, ga * am, -ap, F, fr, ur);
+  F[KVX + DIR - 1] = fma(ga * ap, fma(am, ul, fl), ga * am * fma(-ap, ur, fr));
 }
 #endif
 
-// the five-point stencil of one variable with boundary codes of its own
-// (differing between variables, or extrapolation): out of line
-struct Stencil5 {
-  double f[5];
+// the m values from cell c - 2 on of one variable with boundary codes of its
+// own (differing between variables, or extrapolation): out of line
+struct Stencil6 {
+  double f[6];
 };
-static __device__ __noinline__ Stencil5 stencil_general(const double* __restrict__ a, size_t base, long long stride,
-                                                        int n, int c, int code_l, int code_r) {
-  Stencil5 r;
+static __device__ __noinline__ Stencil6 stencil_general(const double* __restrict__ a, size_t base, long long stride,
+                                                        int n, int c, int m, int code_l, int code_r) {
+  Stencil6 r;
 #pragma unroll 1
-  for (int q = 0; q < 5; q++) r.f[q] = ghost_val(a, base, stride, n, c - 2 + q, code_l, code_r);
+  for (int q = 0; q < m; q++) r.f[q] = ghost_val(a, base, stride, n, c - 2 + q, code_l, code_r);
   return r;
 }
 
@@ -246,34 +294,121 @@ static __device__ __noinline__ void fix_states(const FaceArgs& A, const Metric& 
   }
 }
 
+// The flux of the face above cell c of a pencil (base, stride) from its states
+// wl, wr (variable k at k * C; changed in place by the fix-ups and the GLM
+// upwinding): writes A.F (and A.WD), the signal speed into amax.
+template <int KIND, int DIR, int C>
+__device__ __forceinline__ void face_one(const FaceArgs& A, const Metric& M, unsigned base, unsigned stride, int n,
+                                         int c, int ta, int tb, double* wl, double* wr, double& amax) {
+  typedef Traits<KIND> T;
+  constexpr int NV = T::NV;
+  const Grid& g = A.g;
+  amax = 0.;
+  const size_t nfaces = faces_of<DIR>(g);
+  const unsigned fid = DIR == 0   ? ((unsigned)tb * (unsigned)g.ny + (unsigned)ta) * (unsigned)(g.nx + 1) + (unsigned)c
+                       : DIR == 1 ? ((unsigned)tb * (unsigned)(g.ny + 1) + (unsigned)c) * (unsigned)g.nx + (unsigned)ta
+                                  : (unsigned)c * stride + base;
+  if (T::VISC) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      A.WD[(size_t)q * nfaces + fid] = wl[(NV + q) * C];
+      A.WD[(size_t)(4 + q) * nfaces + fid] = wr[(NV + q) * C];
+    }
+  }
+  const double ch = A.sc->glm_ch_old;
+  double F[NV];
+  int err;
+#ifdef ECHO_EXACT
+  double ql[NV], qr[NV], w0[NV];
+#pragma unroll
+  for (int k = 0; k < NV; k++) {
+    ql[k] = T::VISC && k == KPIZZ && A.P.obtained_zz ? 0. : wl[k * C];
+    qr[k] = T::VISC && k == KPIZZ && A.P.obtained_zz ? 0. : wr[k * C];
+    w0[k] = 0.;
+  }
+#pragma unroll 1
+  for (int k = KVX; k <= KPR; k++)
+    w0[k] = ghost_val(A.v + (size_t)k * g.ncell, base, stride, n, c, A.bc.c[k][0], A.bc.c[k][1]);
+  err = face_tail<KIND, DIR>(A.P, M, ch, ql, qr, w0, F, amax);
+#else
+  {
+    const double lv = wl[KVX * C] * wl[KVX * C] + wl[KVY * C] * wl[KVY * C] + M.g3 * (wl[KVZ * C] * wl[KVZ * C]);
+    const double rv = wr[KVX * C] * wr[KVX * C] + wr[KVY * C] * wr[KVY * C] + M.g3 * (wr[KVZ * C] * wr[KVZ * C]);
+    if (wl[KPR * C] <= 0 || wr[KPR * C] <= 0 || lv >= 1. || rv >= 1.)
+      fix_states<KIND>(A, M, base, stride, n, c, wl, wr, C);
+  }
+  if (T::GLM) {
+    // work_glm[xyz]: psi and the normal B of the face (the second's
+    // correction has the factor psi_r - psi_l, which is zero by then)
+    const int kb = KBX + DIR;
+    const double bl = wl[kb * C], br = wr[kb * C];
+    const double psi = 0.5 * ((wl[T::KG * C] + wr[T::KG * C]) - (br - bl) * ch), bn = 0.5 * (bl + br);
+    wl[T::KG * C] = psi;
+    wr[T::KG * C] = psi;
+    wl[kb * C] = bn;
+    wr[kb * C] = bn;
+  }
+  FaceSide L, R;
+  double vflp, vflm, vfrp, vfrm;
+  err = side_speeds<KIND, DIR + 1>(A.P, M, wl, C, L, vflp, vflm);
+  if (!err) err = side_speeds<KIND, DIR + 1>(A.P, M, wr, C, R, vfrp, vfrm);
+  if (!err) {
+    double ap = 0., am = 0.;
+    if (vflp > ap) ap = vflp;
+    if (vfrp > ap) ap = vfrp;
+    if (-vflm > am) am = -vflm;
+    if (-vfrm > am) am = -vfrm;
+    amax = ap > am ? ap : am;
+    hll_flux<KIND, DIR + 1>(A.P, M, wl, wr, C, L, R, ap, am, F);
+  }
+#endif
+  if (err) {
+    amax = 0.;
+    const size_t cell = base + (size_t)((c >= 1 ? c : 1) - 1) * stride;
+    atomicMin(&A.sc->err_key, ((unsigned long long)cell << 20) | (unsigned long long)err);
+#pragma unroll
+    for (int k = 0; k < NV; k++) F[k] = 0.0;
+  }
+#pragma unroll
+  for (int k = 0; k < NV; k++) *(double*)((char*)(A.F + (size_t)k * nfaces) + 8u * fid) = F[k];
+  if (!err) {
+    // GLM speed of the reference: the last face of the last pencil (work.f90:217,310,401)
+    const int na = DIR == 0 ? g.ny : g.nx, nb = DIR == 2 ? g.ny : g.nz;
+    if (c == n && ta == na - 1 && tb == nb - 1) A.sc->aflux[DIR] = amax;
+  }
+}
+
 // One tile of the sweep along DIR; returns the largest signal speed of this
-// thread's faces.  Called by every thread of the block; blockDim.x is a
-// multiple of the tile's cells: the further groups of threads share the
-// variables of phase 1.  sm: tile_smem<KIND>(lc) bytes.
-template <int KIND, int DIR, int REC, int LC, int NG>
+// thread's faces.  Called by every thread of the block: NG groups of C / CPT
+// threads, the groups sharing the variables of phase 1.  sm:
+// tile_smem<KIND>(LC) bytes.
+template <int KIND, int DIR, int REC, int LC, int CPT, int NG>
 __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, int lw, double* sm) {
   typedef Traits<KIND> T;
-  constexpr int NV = T::NV, C = 1 << LC, UNROLL = ECHO_SWEEP_UNROLL;
+  constexpr int NV = T::NV, C = 1 << LC, NT = C / CPT, NS = CPT + 4, UNROLL = ECHO_SWEEP_UNROLL;
   const Grid& g = A.g;
-  const int slot = threadIdx.x & (C - 1), grp = threadIdx.x >> LC;
+  const int t = NG > 1 ? (int)threadIdx.x & (NT - 1) : (int)threadIdx.x;
+  const int grp = NG > 1 ? (int)threadIdx.x / NT : 0;
   const int n = DIR == 0 ? g.nx : DIR == 1 ? g.ny : g.nz;
   const int W = DIR == 0 ? 1 : 1 << lw;
+  // cell j of thread t is slot j NT + t (the shared accesses of a warp are
+  // consecutive)
   double* plus = sm;                                       // upper face state of a cell
   double* minus = sm + tile_rows_of_states<KIND>() * C;    // its lower face state
-  const Metric M = make_metric(A.coordinates, A.sc->t, A.sc->t3);
+  const double mt = A.sc->t, mt3 = A.sc->t3;
 
-  // this thread's cell: pencil index c (0 and n + 1 are the ghosts next to the
-  // grid), first cell and stride of its pencil, transverse position.  Cell and
-  // face indices are below 2^29 (their doubles' byte offsets below 2^32): the
-  // arrays of a larger grid do not fit the device.
+  // this thread's first cell: pencil index c (0 and n + 1 are the ghosts next
+  // to the grid), first cell and stride of its pencil, transverse position.
+  // Cell and face indices are below 2^29 (their doubles' byte offsets below
+  // 2^32): the arrays of a larger grid do not fit the device.
   int c, ta, tb;
   unsigned base;
   bool ok;
   const unsigned stride = DIR == 0 ? 1u : DIR == 1 ? (unsigned)g.nx : (unsigned)g.nx * (unsigned)g.ny;
   if (DIR == 0) {
-    const unsigned e = tile * (unsigned)(C - 1) + (unsigned)slot;
+    const unsigned e = tile * (unsigned)(C - 2) + (unsigned)(t * CPT);
     const unsigned pen = fast_div(e, g.dnx2);
-    c = (int)(e - pen * (unsigned)(g.nx + 2));
+    c = (int)(e - pen * (((unsigned)g.nx + 3u) & ~1u));
     tb = (int)fast_div(pen, g.dny);
     ta = (int)(pen - (unsigned)tb * (unsigned)g.ny);
     ok = tb < g.nz;
@@ -282,27 +417,30 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
     const unsigned cols = (unsigned)g.nx * (unsigned)(DIR == 1 ? g.nz : g.ny);
     const unsigned nct = (cols + (unsigned)W - 1) >> lw;
     const unsigned rt = tile / nct, ct = tile - rt * nct;
-    const unsigned p = (ct << lw) + (unsigned)(slot & (W - 1));
+    const unsigned p = (ct << lw) + (unsigned)(t & (W - 1));
     tb = (int)fast_div(p, g.dnx);
     ta = (int)(p - (unsigned)tb * (unsigned)g.nx);
-    c = (int)(rt * (unsigned)((C >> lw) - 1)) + (slot >> lw);
-    ok = p < cols && c <= n + 1;
+    c = (int)(rt * (unsigned)((C >> lw) - 1)) + (t >> lw) * CPT;
+    ok = p < cols;
     base = DIR == 1 ? (unsigned)tb * (unsigned)(g.ny * g.nx) + (unsigned)ta : p;
   }
+  ok = ok && c <= n + 1;
 
   if (ok) {
-    // byte offsets of the stencil c-2..c+2, with the ghost fill of evolve_bc[xyz]
-    unsigned off[5];
+    // byte offsets of the stencil from cell c - 2 on, with the ghost fill of
+    // evolve_bc[xyz]; the last cell's own upper neighbour is not read
+    const int last = c + CPT - 1 <= n + 1 ? NS - 1 : NS - 2;
+    unsigned off[NS];
     int neg = 0;
-    if (c >= 3 && c <= n - 2) {
+    if (c >= 3 && c + CPT + 1 <= n) {
 #pragma unroll
-      for (int q = 0; q < 5; q++) off[q] = 8u * (base + (unsigned)(c - 3 + q) * stride);
+      for (int q = 0; q < NS; q++) off[q] = 8u * (base + (unsigned)(c - 3 + q) * stride);
     } else {
 #pragma unroll
-      for (int q = 0; q < 5; q++) {
+      for (int q = 0; q < NS; q++) {
         int qq;
         double sg;
-        map_ghost(c - 2 + q, n, A.bc.c[0][0], A.bc.c[0][1], qq, sg);
+        map_ghost(c - 2 + (q < last ? q : last), n, A.bc.c[0][0], A.bc.c[0][1], qq, sg);
         off[q] = 8u * (base + (unsigned)(qq - 1) * stride);
         if (sg < 0.) neg |= 1 << q;
       }
@@ -311,143 +449,104 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
       const char* vk = (const char*)(A.v + (size_t)k * g.ncell);
       if (A.bc_uniform) {
 #pragma unroll
-        for (int q = 0; q < 5; q++) f[q] = __ldg((const double*)(vk + off[q]));
+        for (int q = 0; q < NS; q++) f[q] = __ldg((const double*)(vk + off[q]));
         if (A.bc_signed) {
 #pragma unroll
-          for (int q = 0; q < 5; q++) f[q] = (neg >> q) & 1 ? -f[q] : f[q];
+          for (int q = 0; q < NS; q++) f[q] = (neg >> q) & 1 ? -f[q] : f[q];
         }
       } else {
-        const Stencil5 s = stencil_general((const double*)vk, base, stride, n, c, A.bc.c[k][0], A.bc.c[k][1]);
+        const Stencil6 s = stencil_general((const double*)vk, base, stride, n, c, last + 1, A.bc.c[k][0], A.bc.c[k][1]);
 #pragma unroll
-        for (int q = 0; q < 5; q++) f[q] = s.f[q];
+        for (int q = 0; q < NS; q++) f[q] = q <= last ? s.f[q] : s.f[q - 1];
+      }
+    };
+    auto put = [&](int k, const double* f) {
+      double pl[CPT], mi[CPT];
+      recon_cells<REC, CPT>(A.P.recal, f, pl, mi);
+#pragma unroll
+      for (int j = 0; j < CPT; j++) {
+        plus[k * C + j * NT + t] = pl[j];
+        minus[k * C + j * NT + t] = mi[j];
       }
     };
     // pi^{eta eta} of a face state follows from the others (derived_pi_zz)
     const int nr = T::VISC && A.P.obtained_zz ? NV - 1 : NV;
-    int k = NG > 1 ? grp : 0;
+    int k = grp;
 #pragma unroll UNROLL
     for (; k < nr; k += NG) {
-      double f[5], pl, mi;
+      double f[NS];
       load(k, f);
-      recon_cell<REC>(A.P.recal, f, pl, mi);
-      plus[k * C + slot] = pl;
-      minus[k * C + slot] = mi;
+      put(k, f);
     }
     // u^mu for the viscous derivatives (work_rec(n,1,4,1)), by the group
     // whose turn it is
     if (T::VISC && k == nr) {
-      double vx[5], vy[5], vz[5], gg[5];
+      const double g3 = A.coordinates == ECHO_BJORKEN ? mt * mt : 1.;
+      double vx[NS], vy[NS], vz[NS], gg[NS];
       load(KVX, vx);
       load(KVY, vy);
       load(KVZ, vz);
 #pragma unroll
-      for (int q = 0; q < 5; q++) {
+      for (int q = 0; q < NS; q++) {
 #ifdef ECHO_EXACT
-        gg[q] = 1. / sqrt(1. - vx[q] * vx[q] - vy[q] * vy[q] - M.g3 * (vz[q] * vz[q]));
+        gg[q] = 1. / sqrt(1. - vx[q] * vx[q] - vy[q] * vy[q] - g3 * (vz[q] * vz[q]));
 #else
-        gg[q] = rsqrt_h3(1. - vx[q] * vx[q] - vy[q] * vy[q] - M.g3 * (vz[q] * vz[q]));
+        gg[q] = rsqrt_h3(1. - vx[q] * vx[q] - vy[q] * vy[q] - g3 * (vz[q] * vz[q]));
 #endif
         vx[q] = gg[q] * vx[q];
         vy[q] = gg[q] * vy[q];
         vz[q] = gg[q] * vz[q];
       }
-      recon_cell<REC>(A.P.recal, gg, plus[(NV + 0) * C + slot], minus[(NV + 0) * C + slot]);
-      recon_cell<REC>(A.P.recal, vx, plus[(NV + 1) * C + slot], minus[(NV + 1) * C + slot]);
-      recon_cell<REC>(A.P.recal, vy, plus[(NV + 2) * C + slot], minus[(NV + 2) * C + slot]);
-      recon_cell<REC>(A.P.recal, vz, plus[(NV + 3) * C + slot], minus[(NV + 3) * C + slot]);
+      put(NV + 0, gg);
+      put(NV + 1, vx);
+      put(NV + 2, vy);
+      put(NV + 3, vz);
     }
   }
   __syncthreads();
 
-  // the face between cell c and the next one of its pencil
+  // the faces above this thread's cells
   double amax = 0.;
-  if (grp == 0 && ok && slot < C - W && c <= n) {
-    const size_t nfaces = faces_of<DIR>(g);
-    const unsigned fid = DIR == 0   ? ((unsigned)tb * (unsigned)g.ny + (unsigned)ta) * (unsigned)(g.nx + 1) + (unsigned)c
-                         : DIR == 1 ? ((unsigned)tb * (unsigned)(g.ny + 1) + (unsigned)c) * (unsigned)g.nx + (unsigned)ta
-                                    : (unsigned)c * stride + base;
-    double* wl = plus + slot;
-    double* wr = minus + slot + W;
-    if (T::VISC) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        A.WD[(size_t)q * nfaces + fid] = wl[(NV + q) * C];
-        A.WD[(size_t)(4 + q) * nfaces + fid] = wr[(NV + q) * C];
-      }
-    }
-    const double ch = A.sc->glm_ch_old;
-    double F[NV];
-    int err;
-#ifdef ECHO_EXACT
-    double ql[NV], qr[NV], w0[NV];
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      ql[k] = T::VISC && k == KPIZZ && A.P.obtained_zz ? 0. : wl[k * C];
-      qr[k] = T::VISC && k == KPIZZ && A.P.obtained_zz ? 0. : wr[k * C];
-      w0[k] = 0.;
-    }
+  const Metric M = make_metric(A.coordinates, mt, mt3);
 #pragma unroll 1
-    for (int k = KVX; k <= KPR; k++)
-      w0[k] = ghost_val(A.v + (size_t)k * g.ncell, base, stride, n, c, A.bc.c[k][0], A.bc.c[k][1]);
-    err = face_tail<KIND, DIR>(A.P, M, ch, ql, qr, w0, F, amax);
-#else
-    {
-      const double lv = wl[KVX * C] * wl[KVX * C] + wl[KVY * C] * wl[KVY * C] + M.g3 * (wl[KVZ * C] * wl[KVZ * C]);
-      const double rv = wr[KVX * C] * wr[KVX * C] + wr[KVY * C] * wr[KVY * C] + M.g3 * (wr[KVZ * C] * wr[KVZ * C]);
-      if (wl[KPR * C] <= 0 || wr[KPR * C] <= 0 || lv >= 1. || rv >= 1.)
-        fix_states<KIND>(A, M, base, stride, n, c, wl, wr, C);
-    }
-    if (T::GLM) {
-      // work_glm[xyz]: psi and the normal B of the face (the second's
-      // correction has the factor psi_r - psi_l, which is zero by then)
-      const int kb = KBX + DIR;
-      const double bl = wl[kb * C], br = wr[kb * C];
-      const double psi = 0.5 * ((wl[T::KG * C] + wr[T::KG * C]) - (br - bl) * ch), bn = 0.5 * (bl + br);
-      wl[T::KG * C] = psi;
-      wr[T::KG * C] = psi;
-      wl[kb * C] = bn;
-      wr[kb * C] = bn;
-    }
-    FaceSide L, R;
-    double vflp, vflm, vfrp, vfrm;
-    err = side_speeds<KIND, DIR + 1>(A.P, M, wl, C, L, vflp, vflm);
-    if (!err) err = side_speeds<KIND, DIR + 1>(A.P, M, wr, C, R, vfrp, vfrm);
-    if (!err) {
-      double ap = 0., am = 0.;
-      if (vflp > ap) ap = vflp;
-      if (vfrp > ap) ap = vfrp;
-      if (-vflm > am) am = -vflm;
-      if (-vfrm > am) am = -vfrm;
-      amax = ap > am ? ap : am;
-      const double a1 = M.gp * (ap == 0. && am == 0. ? 1. : rcp_h3(ap + am));
-#pragma unroll
-      for (int k = 0; k < NV; k++) F[k] = 0.;
-      side_flux<KIND, DIR + 1>(A.P, M, wl, C, L, a1 * ap, am, F);
-      side_flux<KIND, DIR + 1>(A.P, M, wr, C, R, a1 * am, -ap, F);
-    }
-#endif
-    if (err) {
-      amax = 0.;
-      const size_t cell = base + (size_t)((c >= 1 ? c : 1) - 1) * stride;
-      atomicMin(&A.sc->err_key, ((unsigned long long)cell << 20) | (unsigned long long)err);
-#pragma unroll
-      for (int k = 0; k < NV; k++) F[k] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < NV; k++) *(double*)((char*)(A.F + (size_t)k * nfaces) + 8u * fid) = F[k];
-    if (!err) {
-      // GLM speed of the reference: the last face of the last pencil (work.f90:217,310,401)
-      const int na = DIR == 0 ? g.ny : g.nx, nb = DIR == 2 ? g.ny : g.nz;
-      if (c == n && ta == na - 1 && tb == nb - 1) A.sc->aflux[DIR] = amax;
-    }
+  for (int j = 0; j < CPT; j++) {
+    // the cell above is this thread's next one or the first of the thread W
+    // further on; the last pair of an x tile is the first of the next
+    const bool own = CPT > 1 && j < CPT - 1;
+    const int cf = c + j;
+    if (!(grp == 0 && ok && cf <= n && (own ? DIR > 0 || t < NT - 1 : t + W < NT - (DIR == 0 && CPT == 1 ? 1 : 0)))) continue;
+    double* wl = plus + j * NT + t;
+    double* wr = minus + (own ? (j + 1) * NT + t : t + W);
+    double am;
+    face_one<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
+    amax = am > amax ? am : amax;
   }
   return amax;
 }
 
-// threads of a sweep block
-#define ECHO_SWEEP_NT 256
+// Cells of a thread in the large tiles (256 cells): two share loads and
+// differences, but a thread then holds 4 NV doubles of shared memory, which
+// for the twelve variables of the viscous and resistive sets leaves 12 to 16
+// warps an SM; and the limiters of MPE5, the scheme of ideal hydro runs that
+// do not choose, gain nothing from it.  Measured, x / y / eta us a launch:
+// ideal RMHD 97 x 97 x 81 78 / 79 / 84 with one cell, 76 / 70 / 73 with two;
+// resistive 193 x 193 x 129 453 / 496 / 518 with one, 508 / 518 / 547 with
+// two; ideal hydro MPE5 75 x 67 x 49 33 / 27 / 32 with one, 35 / 28 / 36 with two.
+template <int KIND>
+__host__ __device__ constexpr int sweep_cpt(int lc) {
+  return lc == 8 && (KIND == KIND_MHD || KIND == KIND_MHDGLM) ? 2 : 1;
+}
+// threads of a block; the small tiles' (32 cells) are eight groups
+template <int KIND>
+__host__ __device__ constexpr int sweep_threads(int lc) {
+  return 256 / sweep_cpt<KIND>(lc);
+}
+// blocks of an SM: the register bound that was fastest
 #ifndef ECHO_SWEEP_MINB
-#define ECHO_SWEEP_MINB 4
+#define ECHO_SWEEP_MINB 6
+#endif
+#ifndef ECHO_SWEEP_MINB_HD
+#define ECHO_SWEEP_MINB_HD 4
 #endif
 #ifndef ECHO_SWEEP_MINB_VISC
 #define ECHO_SWEEP_MINB_VISC 3
@@ -455,29 +554,35 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
 #ifndef ECHO_SWEEP_MINB_RES
 #define ECHO_SWEEP_MINB_RES 4
 #endif
-#define ECHO_SWEEP_BOUNDS(KIND)                                                          \
-  __launch_bounds__(ECHO_SWEEP_NT, (KIND) == KIND_VISC  ? ECHO_SWEEP_MINB_VISC       \
-                                   : (KIND) == KIND_RES ? ECHO_SWEEP_MINB_RES : ECHO_SWEEP_MINB)
+template <int KIND>
+constexpr int sweep_minb(int lc) {
+  return lc != 8             ? 3
+         : KIND == KIND_HD   ? ECHO_SWEEP_MINB_HD
+         : KIND == KIND_VISC ? ECHO_SWEEP_MINB_VISC
+         : KIND == KIND_RES  ? ECHO_SWEEP_MINB_RES
+                             : ECHO_SWEEP_MINB;
+}
 
 // The sweeps of a stage in one launch: the blocks of the directions one after
 // another, so that the partial last wave of one overlaps the next.  They are
 // independent: each writes its own face fluxes and signal-speed slots.
 template <int KIND, int REC, int LC>
-__global__ void ECHO_SWEEP_BOUNDS(KIND) sweep_kernel(const __grid_constant__ SweepArgs S) {
+__global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC)) sweep_kernel(const __grid_constant__ SweepArgs S) {
   extern __shared__ double sm[];
-  __shared__ double red[ECHO_SWEEP_NT / 32];
+  constexpr int CPT = sweep_cpt<KIND>(LC), NG = (sweep_threads<KIND>(LC) * CPT) >> LC;
+  __shared__ double red[sweep_threads<KIND>(LC) / 32];
   const unsigned b = blockIdx.x;
   double amax;
   int dir;
   if (b < S.first[1]) {
     dir = 0;
-    amax = face_tile<KIND, 0, REC, LC, (ECHO_SWEEP_NT >> LC)>(S.A[0], b, S.lw, sm);
+    amax = face_tile<KIND, 0, REC, LC, CPT, NG>(S.A[0], b, S.lw, sm);
   } else if (b < S.first[2]) {
     dir = 1;
-    amax = face_tile<KIND, 1, REC, LC, (ECHO_SWEEP_NT >> LC)>(S.A[1], b - S.first[1], S.lw, sm);
+    amax = face_tile<KIND, 1, REC, LC, CPT, NG>(S.A[1], b - S.first[1], S.lw, sm);
   } else {
     dir = 2;
-    amax = face_tile<KIND, 2, REC, LC, (ECHO_SWEEP_NT >> LC)>(S.A[2], b - S.first[2], S.lw, sm);
+    amax = face_tile<KIND, 2, REC, LC, CPT, NG>(S.A[2], b - S.first[2], S.lw, sm);
   }
   block_max_atomic(amax, &S.A[0].sc->amax_bits[dir], red);
 }

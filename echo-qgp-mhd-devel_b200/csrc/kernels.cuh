@@ -61,8 +61,8 @@ struct Grid {
   int nx, ny, nz;
   size_t ncell;
   double ddx, ddy, ddz;
-  // division by nx, ny, nx + 1, ny + 1 and nx + 2 of face and cell indices
-  // below 2^32 (set_grid_div)
+  // division by nx, ny, nx + 1, ny + 1 and the even number of cells of a pencil
+  // with its two ghosts, of face and cell indices below 2^32 (set_grid_div)
   FastDiv dnx, dny, dnx1, dny1, dnx2;
 };
 __host__ __device__ inline void set_grid_div(Grid& g) {
@@ -70,7 +70,7 @@ __host__ __device__ inline void set_grid_div(Grid& g) {
   g.dny = make_fastdiv((unsigned)g.ny);
   g.dnx1 = make_fastdiv((unsigned)g.nx + 1u);
   g.dny1 = make_fastdiv((unsigned)g.ny + 1u);
-  g.dnx2 = make_fastdiv((unsigned)g.nx + 2u);
+  g.dnx2 = make_fastdiv(((unsigned)g.nx + 3u) & ~1u);
 }
 
 // boundary codes for one sweep direction: bc[k][side]
@@ -137,9 +137,10 @@ __device__ __forceinline__ void map_ghost(int j, int n, int cl, int cr, int& q, 
 // The face and update kernels are latency-bound (long-scoreboard and
 // dependent FP64 stalls): more resident warps win over the spills a lower
 // register cap costs.  Measured on B200 (blocks of 128 per SM): faces 7
-// (ideal RMHD; 5 is 10 % slower) and 5 (viscous; 3 is 15 % slower); update
-// 7 (ideal RMHD, from 4 uncapped), 5 (viscous, from 2) and 6 with the
-// learned seed (from 2: 0.74 vs 1.17 ms per step).
+// (ideal RMHD; 5 is 10 % slower) and 5 (viscous; 3 is 15 % slower; both the
+// batched sweeps); update 6 (ideal RMHD: 307 us a step; 5 319, 7 308, 8 352),
+// 5 (viscous, from 2) and 6 with the learned seed (from 2: 0.74 vs 1.17 ms
+// per step).
 #ifndef ECHO_FACE_MINB
 #define ECHO_FACE_MINB 7
 #endif
@@ -156,7 +157,7 @@ __device__ __forceinline__ void map_ghost(int j, int n, int cl, int cr, int& q, 
   __launch_bounds__(128, (KIND) == KIND_VISC  ? ECHO_FACE_MINB_VISC              \
                          : (KIND) == KIND_RES ? ECHO_FACE_MINB_RES : ECHO_FACE_MINB)
 #ifndef ECHO_UPDATE_MINB
-#define ECHO_UPDATE_MINB 7
+#define ECHO_UPDATE_MINB 6
 #endif
 #ifndef ECHO_UPDATE_MINB_VISC
 #define ECHO_UPDATE_MINB_VISC 5
@@ -670,19 +671,19 @@ __device__ __forceinline__ void mlp_seed(const MlpDev& net, const Metric& M, boo
 // combination or writes du (MODE_RHS), then con2prim.  update_cell reads
 // the face fluxes of the three sweep kernels; the fused stage kernel
 // computes them itself (stage.cuh).
-template <int KIND, bool SEED, bool IMEX = false>
+template <int KIND, bool SEED, bool IMEX, int ALGO>
 __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, bool active, int ix, int iy, int iz,
                                               double* du, double* dv) {
   typedef Traits<KIND> T;
   const int NV = T::NV;
   const Grid& g = A.g;
-  unsigned long long my_iters = 0, my_fallbacks = 0, my_brackets = 0;
+  unsigned my_iters = 0, my_fallbacks = 0, my_brackets = 0;
   const Metric M = make_metric(A.coordinates, A.sc->t, A.sc->t3);
   double vv[NV], uu[NV];
   if (active) {
     double src[NV], kap[2] = {0., 0.};
 #pragma unroll
-    for (int k = 0; k < NV; k++) vv[k] = A.vin[(size_t)k * g.ncell + c];
+    for (int k = 0; k < NV; k++) vv[k] = *(const double*)((const char*)(A.vin + (size_t)k * g.ncell) + 8u * (unsigned)c);
     if (T::VISC) {
       if (A.vsnap) {
 #pragma unroll
@@ -702,12 +703,22 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
           vy = A.vnew[2 * g.ncell + c];
           vz = A.vnew[3 * g.ncell + c];
         }
+#ifdef ECHO_EXACT
         double gamma1 = 1. / sqrt(1. - M.g1 * (vxo * vxo) - M.g2 * (vyo * vyo) - A.sc->g3old * (vzo * vzo));
         double gamma2 = 1. / sqrt(1. - M.g1 * (vx * vx) - M.g2 * (vy * vy) - M.g3 * (vz * vz));
         dv[DTT] = (gamma2 - gamma1) / (ti);
         dv[DXT] = (gamma2 * vx - gamma1 * vxo) / ti;
         dv[DYT] = (gamma2 * vy - gamma1 * vyo) / ti;
         dv[DZT] = (gamma2 * vz - gamma1 * vzo) / ti;
+#else
+        const double gamma1 = rsqrt_h3(1. - vxo * vxo - vyo * vyo - A.sc->g3old * (vzo * vzo));
+        const double gamma2 = rsqrt_h3(1. - vx * vx - vy * vy - M.g3 * (vz * vz));
+        const double iti = rcp_h3(ti);
+        dv[DTT] = (gamma2 - gamma1) * iti;
+        dv[DXT] = (gamma2 * vx - gamma1 * vxo) * iti;
+        dv[DYT] = (gamma2 * vy - gamma1 * vyo) * iti;
+        dv[DZT] = (gamma2 * vz - gamma1 * vzo) * iti;
+#endif
       }
     }
     // resistive: charge density d_i E^i by central differences with the
@@ -744,11 +755,11 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
                                     T::RES ? stiff : nullptr);
       if (err) atomicMin(&A.sc->err_key, ((unsigned long long)c << 20) | (unsigned long long)err);
     }
-#pragma unroll
-    for (int k = 0; k < NV; k++) du[k] = du[k] - src[k];
+    const unsigned c8 = 8u * (unsigned)c;  // cell indices are below 2^29 (face_tile)
+    auto at = [&](auto* a, int k) { return (decltype(a))((char*)(a + (size_t)k * g.ncell) + c8); };
     if (A.mode == MODE_RHS) {
 #pragma unroll
-      for (int k = 0; k < NV; k++) A.du_out[(size_t)k * g.ncell + c] = du[k];
+      for (int k = 0; k < NV; k++) *at(A.du_out, k) = du[k] - src[k];
       if (T::RES && A.dus_out) {
 #pragma unroll
         for (int i = 0; i < 3; i++) A.dus_out[(size_t)i * g.ncell + c] = 0. - stiff[i];
@@ -756,26 +767,40 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
     } else {
       // RK combination (evolve.f90:196-201)
       const double dt = A.sc->dt;
+      // all loads of a kind together: each batch is one trip to memory
+      double u0[NV];
+#pragma unroll
+      for (int k = 0; k < NV; k++) uu[k] = *at(A.uin, k);
+      if (A.irk != 1) {
+#pragma unroll
+        for (int k = 0; k < NV; k++) u0[k] = *at(A.u0, k);
+      } else {
+        if (T::GLM) {
+          uu[T::KG] = uu[T::KG] * A.sc->expfact;
+          *at(A.uin, T::KG) = uu[T::KG];  // u0 = u after the GLM half step
+        }
+#pragma unroll
+        for (int k = 0; k < NV; k++) u0[k] = uu[k];
+      }
 #pragma unroll
       for (int k = 0; k < NV; k++) {
-        double ui = A.uin[(size_t)k * g.ncell + c];
-        if (T::GLM && k == T::KG && A.irk == 1) {
-          ui = ui * A.sc->expfact;
-          A.uin[(size_t)k * g.ncell + c] = ui;  // u0 = u after the GLM half step
-        }
-        double u0 = A.irk == 1 ? ui : A.u0[(size_t)k * g.ncell + c];
+        const double ui = uu[k], d = du[k] - src[k];
         if (T::VISC && IMEX && k >= KPIBU) {
           // IMEX RK2/RK3: the relaxation -kap u of the stresses at the new
           // stage value, u_new = u_expl + c2 dt kap (u - u_new)
           double ck = A.c2 * dt * (k == KPIBU ? kap[0] : kap[1]);
-          uu[k] = (A.c1 * u0 + A.c2 * (ui - dt * du[k]) + ck * ui) / (1. + ck);
+#ifdef ECHO_EXACT
+          uu[k] = (A.c1 * u0[k] + A.c2 * (ui - dt * d) + ck * ui) / (1. + ck);
+#else
+          uu[k] = (A.c1 * u0[k] + A.c2 * (ui - dt * d) + ck * ui) * rcp_h3(1. + ck);
+#endif
         } else {
-          uu[k] = A.c1 * u0 + A.c2 * (ui - dt * du[k]);
+          uu[k] = A.c1 * u0[k] + A.c2 * (ui - dt * d);
         }
       }
       if (T::GLM && A.irk == A.nrk) uu[T::KG] = uu[T::KG] * A.sc->expfact;
 #pragma unroll
-      for (int k = 0; k < NV; k++) A.uout[(size_t)k * g.ncell + c] = uu[k];
+      for (int k = 0; k < NV; k++) *at(A.uout, k) = uu[k];
     }
   }
   if (A.mode == MODE_RK) {
@@ -789,103 +814,91 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
     if (active && !(T::MHD && !T::RES && c2p_alt_algo(A.algo))) {  // ALG_SOLV 2..6: c2p_alt_kernel
       // con2prim (evolve_u2v, evolve.f90:789-866)
       int it = 0, sfail = 0;
-      int err = cons2prim<KIND>(A.P, M, A.algo, A.tol, uu, vv, &it, sp, &sfail);
-      my_iters = (unsigned long long)it;
-      my_fallbacks = (unsigned long long)(sfail & 1);
-      my_brackets = (unsigned long long)(sfail >> 1);
+      int err = cons2prim<KIND, false, ALGO>(A.P, M, A.algo, A.tol, uu, vv, &it, sp, &sfail);
+      my_iters = (unsigned)it;
+      my_fallbacks = (unsigned)(sfail & 1);
+      my_brackets = (unsigned)(sfail >> 1);
+      A.fail[c] = err ? 1 : 0;
       if (err) {
-        A.fail[c] = 1;
         atomicAdd(&A.sc->nfail, 1);
       } else {
-        A.fail[c] = 0;
 #pragma unroll
-        for (int k = 0; k < NV; k++) A.vout[(size_t)k * g.ncell + c] = vv[k];
+        for (int k = 0; k < NV; k++) *(double*)((char*)(A.vout + (size_t)k * g.ncell) + 8u * (unsigned)c) = vv[k];
       }
     }
     // per-warp sums of iteration counts, seed and bracketed fallbacks
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      my_iters += __shfl_xor_sync(0xffffffffu, my_iters, o);
-      my_fallbacks += __shfl_xor_sync(0xffffffffu, my_fallbacks, o);
-      my_brackets += __shfl_xor_sync(0xffffffffu, my_brackets, o);
+    my_iters = __reduce_add_sync(0xffffffffu, my_iters);
+    my_fallbacks = __reduce_add_sync(0xffffffffu, my_fallbacks);
+    my_brackets = __reduce_add_sync(0xffffffffu, my_brackets);
+    if ((threadIdx.x & 31) == 0) {
+      if (my_iters) atomicAdd(&A.sc->c2p_iters, (unsigned long long)my_iters);
+      if (my_fallbacks) atomicAdd(&A.sc->fallbacks, (unsigned long long)my_fallbacks);
+      if (my_brackets) atomicAdd(&A.sc->brackets, (unsigned long long)my_brackets);
     }
-    if ((threadIdx.x & 31) == 0 && my_iters) atomicAdd(&A.sc->c2p_iters, my_iters);
-    if ((threadIdx.x & 31) == 0 && my_fallbacks) atomicAdd(&A.sc->fallbacks, my_fallbacks);
-    if ((threadIdx.x & 31) == 0 && my_brackets) atomicAdd(&A.sc->brackets, my_brackets);
   }
 }
 
 
-template <int KIND, bool SEED, bool IMEX = false>
+template <int KIND, bool SEED, bool IMEX = false, int ALGO = C2P_ANY>
 __device__ __forceinline__ void update_cell(const UpdateArgs& A, size_t c, bool active) {
   typedef Traits<KIND> T;
   const int NV = T::NV;
   const Grid& g = A.g;
   int ix = 0, iy = 0, iz = 0;
   double du[NV], dv[NDER];
+  // byte offsets of the cell's lower x, y and eta faces (faces ix, iy, iz of
+  // its pencils); face indices are below 2^29 (face_tile)
+  unsigned fx = 0, fy = 0, fz = 0;
+  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, sy = 8u * nx, sz = 8u * nx * ny;
+  const size_t nfx = faces_of<0>(g), nfy = faces_of<1>(g), nfz = faces_of<2>(g);
+  auto up = [](const double* a, size_t k, unsigned off) { return *(const double*)((const char*)(a + k) + off); };
   if (active) {
-    if (g.ncell < (1ull << 32)) {  // multiply-high divisions (FastDiv)
-      const unsigned cc = (unsigned)c, r = fast_div(cc, g.dnx), q = fast_div(r, g.dny);
-      ix = (int)(cc - r * (unsigned)g.nx);
-      iy = (int)(r - q * (unsigned)g.ny);
-      iz = (int)q;
-    } else {
-      ix = (int)(c % g.nx);
-      size_t r = c / g.nx;
-      iy = (int)(r % g.ny);
-      iz = (int)(r / g.ny);
-    }
-    const size_t nfx = (size_t)(g.nx + 1) * g.ny * g.nz;
-    const size_t nfy = (size_t)g.nx * (g.ny + 1) * g.nz;
-    const size_t nfz = (size_t)g.nx * g.ny * (g.nz + 1);
-    const size_t fx = ((size_t)iz * g.ny + iy) * (g.nx + 1) + ix;       // face ix-1/2 -> index ix
-    const size_t fy = ((size_t)iz * (g.ny + 1) + iy) * g.nx + ix;
-    const size_t fz = ((size_t)iz * g.ny + iy) * g.nx + ix;
-    // flux divergence in the reference's order: du = 0; += x; += y; += z
+    const unsigned cc = (unsigned)c, r = fast_div(cc, g.dnx), q = fast_div(r, g.dny);
+    ix = (int)(cc - r * nx);
+    iy = (int)(r - q * ny);
+    iz = (int)q;
+    fx = 8u * (r * (nx + 1) + (unsigned)ix);
+    fy = 8u * ((q * (ny + 1) + (unsigned)iy) * nx + (unsigned)ix);
+    fz = 8u * cc;
+    // flux divergence in the reference's order, du = 0; += x; += y; += z; the
+    // loads of a direction together, one trip to memory each
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
-      double d = 0.;
-      if (g.nx > 1) d = d + g.ddx * (A.Fx[(size_t)k * nfx + fx + 1] - A.Fx[(size_t)k * nfx + fx]);
-      if (g.ny > 1) d = d + g.ddy * (A.Fy[(size_t)k * nfy + fy + g.nx] - A.Fy[(size_t)k * nfy + fy]);
-      if (g.nz > 1)
-        d = d + g.ddz * (A.Fz[(size_t)k * nfz + fz + (size_t)g.nx * g.ny] - A.Fz[(size_t)k * nfz + fz]);
-      du[k] = d;
-    }
+    for (int k = 0; k < NV; k++) du[k] = 0.;
+    auto flux = [&](const double* F, size_t nf, unsigned f, unsigned s, double dd) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) du[k] = du[k] + dd * (up(F, k * nf, f + s) - up(F, k * nf, f));
+    };
+    if (g.nx > 1) flux(A.Fx, nfx, fx, 8u, g.ddx);
+    if (g.ny > 1) flux(A.Fy, nfy, fy, sy, g.ddy);
+    if (g.nz > 1) flux(A.Fz, nfz, fz, sz, g.ddz);
     if (T::VISC) {
 #pragma unroll
-      for (int q = 0; q < NDER; q++) dv[q] = 0.;
+      for (int i = 0; i < NDER; i++) dv[i] = 0.;
       const int dk[3][4] = {{DTX, DXX, DYX, DZX}, {DTY, DXY, DYY, DZY}, {DTZ, DXZ, DYZ, DZZ}};
+      auto grad = [&](const double* W, size_t nf, unsigned f, unsigned s, int i) {
+        return up(W, i * nf, f + s) + up(W, (4 + i) * nf, f + s) - up(W, i * nf, f) - up(W, (4 + i) * nf, f);
+      };
       if (g.nx > 1) {
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-          dv[dk[0][q]] = g.ddx * 0.5 *
-                         (A.WDx[(size_t)q * nfx + fx + 1] + A.WDx[(size_t)(4 + q) * nfx + fx + 1] -
-                          A.WDx[(size_t)q * nfx + fx] - A.WDx[(size_t)(4 + q) * nfx + fx]);
+        for (int i = 0; i < 4; i++) dv[dk[0][i]] = g.ddx * 0.5 * grad(A.WDx, nfx, fx, 8u, i);
       }
       if (g.ny > 1) {
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-          dv[dk[1][q]] = g.ddy * 0.5 *
-                         (A.WDy[(size_t)q * nfy + fy + g.nx] + A.WDy[(size_t)(4 + q) * nfy + fy + g.nx] -
-                          A.WDy[(size_t)q * nfy + fy] - A.WDy[(size_t)(4 + q) * nfy + fy]);
+        for (int i = 0; i < 4; i++) dv[dk[1][i]] = g.ddy * 0.5 * grad(A.WDy, nfy, fy, sy, i);
       }
       if (g.nz > 1) {
-        size_t s = (size_t)g.nx * g.ny;
 #pragma unroll
-        for (int q = 0; q < 4; q++)
-          dv[dk[2][q]] = g.ddz * 0.5 *
-                         (A.WDz[(size_t)q * nfz + fz + s] + A.WDz[(size_t)(4 + q) * nfz + fz + s] -
-                          A.WDz[(size_t)q * nfz + fz] - A.WDz[(size_t)(4 + q) * nfz + fz]);
+        for (int i = 0; i < 4; i++) dv[dk[2][i]] = g.ddz * 0.5 * grad(A.WDz, nfz, fz, sz, i);
       }
     }
   }
-  update_finish<KIND, SEED, IMEX>(A, c, active, ix, iy, iz, du, dv);
+  update_finish<KIND, SEED, IMEX, ALGO>(A, c, active, ix, iy, iz, du, dv);
 }
 
-template <int KIND, bool SEED, bool IMEX = false>
-__global__ void ECHO_UPDATE_BOUNDS(KIND, SEED) update_kernel(UpdateArgs A) {
+template <int KIND, bool SEED, bool IMEX = false, int ALGO = C2P_ANY>
+__global__ void ECHO_UPDATE_BOUNDS(KIND, SEED) update_kernel(const __grid_constant__ UpdateArgs A) {
   size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  update_cell<KIND, SEED, IMEX>(A, c, c < A.g.ncell);
+  update_cell<KIND, SEED, IMEX, ALGO>(A, c, c < A.g.ncell);
 }
 
 // ---------------------------------------------------------------------------
@@ -933,29 +946,38 @@ __global__ void __launch_bounds__(128, ECHO_SSP_MINB) ssp_combine_kernel(SspArgs
   double uu[NV], vv[NV];
   const double dt = A.sc->dt;
   if (active) {
+    // the branch on the stage outside the loops, so that a stage's loads go
+    // out together; byte offsets below 2^32 (face_tile)
+    const unsigned c8 = 8u * (unsigned)c;
+    auto at = [&](const double* a, int k) { return *(const double*)((const char*)(a + (size_t)k * g.ncell) + c8); };
+    // stiff right-hand sides: zero but for E of resistive runs
+    auto stiff = [&](const double* a, int k) { return T::RES && k >= KEX && k <= KEZ ? at(a, k - KEX) : 0.0; };
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
-      size_t i = (size_t)k * g.ncell + c;
-      double u0 = A.u0[i];
-      // stiff right-hand sides: zero but for E of resistive runs
-      double s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0;
-      if (T::RES && k >= KEX && k <= KEZ) {
-        size_t j = (size_t)(k - KEX) * g.ncell + c;
-        if (A.stage == 2 || A.stage == 4) s1 = A.ds1[j];
-        if (A.stage >= 3) s2 = A.ds2[j];
-        if (A.stage >= 4) s3 = A.ds3[j];
-        if (A.stage == 5) s4 = A.ds4[j];
-      }
-      if (A.stage == 2) {
-        uu[k] = u0 + dt * alpha_imex * s1;
-      } else if (A.stage == 3) {
-        uu[k] = u0 - dt * (A.du2[i] + (1. - alpha_imex) * s2);
-      } else if (A.stage == 4) {
-        uu[k] = u0 - dt * (A.du2[i] / 4. + A.du3[i] / 4. + beta_imex * s1 + eta_imex * s2 + delta_imex * s3);
-      } else {
-        uu[k] = u0 - dt * (A.du2[i] / 6. + A.du3[i] / 6. + A.du4[i] * 2. / 3. + s2 / 6. + s3 / 6. + s4 * 2. / 3.);
-      }
-      vv[k] = A.vin[i];
+    for (int k = 0; k < NV; k++) vv[k] = at(A.vin, k);
+    if (A.stage == 2) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) uu[k] = at(A.u0, k) + dt * alpha_imex * stiff(A.ds1, k);
+    } else if (A.stage == 3) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) uu[k] = at(A.u0, k) - dt * (at(A.du2, k) + (1. - alpha_imex) * stiff(A.ds2, k));
+    } else if (A.stage == 4) {
+#pragma unroll
+      for (int k = 0; k < NV; k++)
+        uu[k] = at(A.u0, k) - dt * (at(A.du2, k) / 4. + at(A.du3, k) / 4. + beta_imex * stiff(A.ds1, k) +
+                                    eta_imex * stiff(A.ds2, k) + delta_imex * stiff(A.ds3, k));
+    } else {
+#ifdef ECHO_EXACT
+#pragma unroll
+      for (int k = 0; k < NV; k++)
+        uu[k] = at(A.u0, k) - dt * (at(A.du2, k) / 6. + at(A.du3, k) / 6. + at(A.du4, k) * 2. / 3. +
+                                    stiff(A.ds2, k) / 6. + stiff(A.ds3, k) / 6. + stiff(A.ds4, k) * 2. / 3.);
+#else
+      const double dt6 = dt / 6.;  // the weights are 1, 1 and 4 sixths
+#pragma unroll
+      for (int k = 0; k < NV; k++)
+        uu[k] = at(A.u0, k) - dt6 * (at(A.du2, k) + at(A.du3, k) + stiff(A.ds2, k) + stiff(A.ds3, k) +
+                                     4. * (at(A.du4, k) + stiff(A.ds4, k)));
+#endif
     }
     if (T::GLM && A.stage == 5) uu[T::KG] = uu[T::KG] * A.sc->expfact;
 #pragma unroll

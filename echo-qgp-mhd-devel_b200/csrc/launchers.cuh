@@ -10,9 +10,10 @@ namespace echo {
 // ---------------------------------------------------------------------------
 // kernel dispatch
 // ---------------------------------------------------------------------------
-// Tile of the sweeps (faces.cuh): 256 cells, one thread each, where that
-// fills the device; smaller tiles, with the block's further threads sharing the
-// variables, where it does not.
+// Tile of the sweeps (faces.cuh): 256 cells where that gives every SM two
+// blocks; 32 cells, with the block's further threads sharing the variables,
+// where it does not (201 x 201 viscous x / y sweep 28 / 25 us with 32 cells,
+// 25 / 23 with 256; 101 x 101 hydro 12 / 9 and 14 / 12).
 inline int sweep_lc(const EchoCtx* c, int mask) {
   unsigned t = 0;
   for (int d = 0; d < 3; d++)
@@ -49,7 +50,7 @@ void launch_faces(EchoCtx* c, int mask) {
   const size_t smem = tile_smem<KIND>(lc);
   auto go = [&](auto* fn) {
     if (smem > 40 * 1024) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fn<<<blocks, ECHO_SWEEP_NT, smem, c->stream>>>(S);
+    fn<<<blocks, sweep_threads<KIND>(lc), smem, c->stream>>>(S);
   };
   // the schemes in use get a kernel of their own; the others choose at run time
   auto pick = [&](auto big, auto small) { lc == 8 ? go(big) : go(small); };
@@ -115,6 +116,9 @@ void launch_update(EchoCtx* c, int irk, int mode, double* du_out) {
     update_kernel<KIND, CAN_SEED><<<blocks, 128, 0, c->stream>>>(A);
   else if (Traits<KIND>::VISC && c->p.imex && mode == MODE_RK)
     update_kernel<KIND, false, Traits<KIND>::VISC><<<blocks, 128, 0, c->stream>>>(A);
+  else if (Traits<KIND>::MHD && !Traits<KIND>::RES && A.algo == ECHO_C2P_NEWTON && mode == MODE_RK)
+    update_kernel<KIND, false, false, Traits<KIND>::MHD && !Traits<KIND>::RES ? C2P_NEWTON : C2P_ANY>
+        <<<blocks, 128, 0, c->stream>>>(A);
   else
     update_kernel<KIND, false><<<blocks, 128, 0, c->stream>>>(A);
   if (Traits<KIND>::MHD && !Traits<KIND>::RES && mode == MODE_RK && c2p_alt_algo(A.algo))

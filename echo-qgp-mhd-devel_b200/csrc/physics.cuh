@@ -59,6 +59,22 @@ enum { KEX = 8, KEY = 9, KEZ = 10 };              // resistive E^i
 // derivative indices (common.f90:70-71), 0-based
 enum { DTX = 0, DTY, DTZ, DXX, DXY, DXZ, DYX, DYY, DYZ, DZX, DZY, DZZ, DTT, DXT, DYT, DZT, NDER = 16 };
 
+// One interval of the EoS table, rows i and i + 1: everything a lookup in it
+// reads, in one 64-byte line (the columns are 2048 entries apart).  e(p) from
+// the first half, p(e) from te, tp and the third quarter, c_s^2 the last.
+struct __align__(16) EosRec {
+  double tp, te;     // p, e of row i
+  double sl_ep, tp1; // de/dp; p of row i + 1
+  double sl_pe, te1; // dp/de = (dp/dT) / (de/dT); e of row i + 1
+  double tc, sl_ce;  // c_s^2 of row i; d(c_s^2)/de
+};
+// A bucket of the bracket search (tab_bracket): the lower bound h of the
+// bracket of its values and the table value h stands for
+struct __align__(16) EosBucket {
+  double node;
+  int h, pad;
+};
+
 // Parameters and per-step metric, passed by value to every kernel.
 struct DevPhys {
   int eqstate, coordinates, recal, obtained_zz, init_type, bulkvis;
@@ -72,11 +88,13 @@ struct DevPhys {
   const int* __restrict__ bkp;
   long long bke0, bkp0;
   int nbke, nbkp;
-  // product build: slopes of every table interval, de/dp, d(c_s^2)/de and
-  // dp/de (null: interpolate with divisions, as the reference does)
-  const double* __restrict__ sl_ep;
-  const double* __restrict__ sl_ce;
-  const double* __restrict__ sl_pe;
+  // product build: the intervals of the table as records and the buckets of
+  // their bracket search (null: search the columns and interpolate with
+  // divisions, as the reference does); the table's first and last e and p
+  const struct EosRec* __restrict__ rec;
+  const struct EosBucket* __restrict__ qe;
+  const struct EosBucket* __restrict__ qp;
+  double emin, emax, pmin, pmax;
   double maxspeed, eta_over_s, tau_pi_coeff, enezero, przero, glm_alpha;
   double sigma_el, sigma_chiral;  // resistive runs: conductivities (code units)
 };
@@ -150,8 +168,13 @@ __device__ __forceinline__ double rsqrt_h3(double a) {
 }
 // sqrt(a); arguments below 1e-290 (zero: a state without sound) give 0
 __device__ __forceinline__ double sqrt_h3(double a) {
-  const double r = a * rsqrt_h3(a);
-  return fabs(a) < 1e-290 ? 0. : r;
+  const double y = rsqrt_h3(a), r = a * y;
+  return fabs(a) < 1e-290 ? 0. : fma(fma(-r, r, a), 0.5 * y, r);
+}
+// b / a, the quotient of rcp_h3 corrected by its residual
+__device__ __forceinline__ double div_h3(double b, double a) {
+  const double x = rcp_h3(a), q = b * x;
+  return fma(fma(-q, a, b), x, q);
 }
 #endif
 
@@ -189,21 +212,87 @@ __device__ __forceinline__ int tab_bracket(const double* __restrict__ arr, const
   while (h < n && __ldg(arr + h - 1) < val) h++;
   return h;
 }
+#ifdef ECHO_EXACT
+struct EosAt {
+  int h;
+};
+#else
+// Product build: the interval of a lookup.  The bracket is tab_search's (the
+// smallest row h >= 2 with arr(h) >= val), found with two dependent loads --
+// the bucket, then the record, which holds the values that confirm it -- where
+// bucket, scan and columns took four: the lookups of the fluxes and of the
+// con2prim Newton loops are latency.  Kept across the steps of a Newton
+// iteration: an interval that still holds the value is not looked up again.
+struct EosAt {
+  double p0, e0, sl;  // row i; slope of the looked-up direction
+  double hi;          // upper end of the interval in the looked-up variable
+  int h;              // bracket (rows h - 1, h; 1-based), 0 = none yet
+};
+__device__ __forceinline__ int eos_bucket(const EosBucket* __restrict__ q, long long k0, int nb, int n, double val) {
+  long long key = (__double_as_longlong(val) >> BK_SHIFT) - k0;
+  key = key < 0 ? 0 : (key >= nb ? nb - 1 : key);
+  const double2 b = __ldg((const double2*)(q + key));
+  const int h = __double2loint(b.y);
+  return h < n && b.x < val ? h + 1 : h;
+}
+// interval of the p column that holds pr (pmin <= pr <= pmax)
+__device__ __forceinline__ void eos_at_p(const DevPhys& P, double pr, EosAt& a) {
+  int h = eos_bucket(P.qp, P.bkp0, P.nbkp, P.nt, pr);
+  const double2* r = (const double2*)(P.rec + (h - 2));
+  double2 x = __ldg(r), y = __ldg(r + 1);
+  while (h < P.nt && y.y < pr) {
+    h++;
+    r += 4;
+    x = __ldg(r);
+    y = __ldg(r + 1);
+  }
+  a.p0 = x.x;
+  a.e0 = x.y;
+  a.sl = y.x;
+  a.hi = y.y;
+  a.h = h;
+}
+// interval of the e column that holds en (emin <= en <= emax)
+__device__ __forceinline__ void eos_at_e(const DevPhys& P, double en, EosAt& a) {
+  int h = eos_bucket(P.qe, P.bke0, P.nbke, P.nt, en);
+  const double2* r = (const double2*)(P.rec + (h - 2));
+  double2 x = __ldg(r), y = __ldg(r + 2);
+  while (h < P.nt && y.y < en) {
+    h++;
+    r += 4;
+    x = __ldg(r);
+    y = __ldg(r + 2);
+  }
+  a.p0 = x.x;
+  a.e0 = x.y;
+  a.sl = y.x;
+  a.hi = y.y;
+  a.h = h;
+}
+// whether the interval of an earlier lookup is the one of val (its lower end lo)
+__device__ __forceinline__ bool eos_holds(const EosAt& a, double lo, double val) {
+  return a.h > 0 && (val > lo || (a.h == 2 && val == lo)) && val <= a.hi;
+}
+#endif
 #define SEARCH_E(P, val) tab_bracket((P).te, (P).bke, (P).bke0, (P).nbke, (P).nt, (val))
 #define SEARCH_P(P, val) tab_bracket((P).tp, (P).bkp, (P).bkp0, (P).nbkp, (P).nt, (val))
 
 // eos_energy: get_energy (eos.f90:468-523) / eos_energy_ana (eos.f90:1104-1185)
 __device__ __forceinline__ int eos_energy(const DevPhys& P, double rh, double* en, double pr) {
   if (P.eqstate == ECHO_EOS_TABLE) {
-    if (pr < __ldg(P.tp)) return 125;
-    if (pr > __ldg(P.tp + P.nt - 1)) return 126;
-    int h = SEARCH_P(P, pr);
 #ifndef ECHO_EXACT
-    if (P.sl_ep) {
-      *en = __ldg(P.te + h - 2) + (pr - __ldg(P.tp + h - 2)) * __ldg(P.sl_ep + h - 2);
+    if (P.rec) {
+      if (pr < P.pmin) return 125;
+      if (pr > P.pmax) return 126;
+      EosAt a;
+      eos_at_p(P, pr, a);
+      *en = a.e0 + (pr - a.p0) * a.sl;
       return 0;
     }
 #endif
+    if (pr < __ldg(P.tp)) return 125;
+    if (pr > __ldg(P.tp + P.nt - 1)) return 126;
+    int h = SEARCH_P(P, pr);
     double p2 = __ldg(P.tp + h - 1), p1 = __ldg(P.tp + h - 2);
     double e2 = __ldg(P.te + h - 1), e1 = __ldg(P.te + h - 2);
     *en = e1 + (e2 - e1) * (pr - p1) / (p2 - p1);
@@ -220,22 +309,36 @@ __device__ __forceinline__ int eos_energy(const DevPhys& P, double rh, double* e
   return 0;
 }
 
+#ifndef ECHO_EXACT
+// p(e) of a table with records; a holds the interval of the last call (h = 0: none)
+__device__ __forceinline__ int eos_pressure_at(const DevPhys& P, double en, double* pr, double* dprdrh,
+                                               double* dprden, EosAt& a) {
+  if (!eos_holds(a, a.e0, en)) {
+    if (en < P.emin) return 123;
+    if (en > P.emax) return 124;
+    eos_at_e(P, en, a);
+  }
+  *pr = a.p0 + (en - a.e0) * a.sl;
+  *dprdrh = 0;
+  *dprden = a.sl;
+  return 0;
+}
+#endif
+
 // eos_pressure: get_pressure (eos.f90:399-464) / eos_pressure_ana (eos.f90:886-922)
 __device__ __forceinline__ int eos_pressure(const DevPhys& P, double rh, double en, double* pr,
                                             double* dprdrh, double* dprden) {
   if (P.eqstate == ECHO_EOS_TABLE) {
+#ifndef ECHO_EXACT
+    if (P.rec) {
+      EosAt a;
+      a.h = 0;
+      return eos_pressure_at(P, en, pr, dprdrh, dprden, a);
+    }
+#endif
     if (en < __ldg(P.te)) return 123;
     if (en > __ldg(P.te + P.nt - 1)) return 124;
     int h = SEARCH_E(P, en);
-#ifndef ECHO_EXACT
-    if (P.sl_pe) {  // dp/de = (dp/dT)/(de/dT) of the interval, precomputed
-      double sl = __ldg(P.sl_pe + h - 2);
-      *pr = __ldg(P.tp + h - 2) + (en - __ldg(P.te + h - 2)) * sl;
-      *dprdrh = 0;
-      *dprden = sl;
-      return 0;
-    }
-#endif
     double p2 = __ldg(P.tp + h - 1), p1 = __ldg(P.tp + h - 2);
     double e2 = __ldg(P.te + h - 1), e1 = __ldg(P.te + h - 2);
     double t2 = __ldg(P.tT + h - 1), t1 = __ldg(P.tT + h - 2);
@@ -261,42 +364,45 @@ __device__ __forceinline__ int eos_pressure(const DevPhys& P, double rh, double 
 }
 
 #ifndef ECHO_EXACT
-// Product build, the face states of system_flux: e(p) interpolated in the p
-// interval of the bracket h (returned for eos_sound_at), with the interval's
-// precomputed slope instead of a division.  h = 0 when the EoS is not a
-// table with slopes (then eos_energy / eos_sound are used).
-__device__ __forceinline__ int eos_energy_h(const DevPhys& P, double rh, double* en, double pr, int* h) {
-  if (P.eqstate == ECHO_EOS_TABLE && P.sl_ep) {
-    if (pr < __ldg(P.tp)) return 125;
-    if (pr > __ldg(P.tp + P.nt - 1)) return 126;
-    int hh = SEARCH_P(P, pr);
-    *en = __ldg(P.te + hh - 2) + (pr - __ldg(P.tp + hh - 2)) * __ldg(P.sl_ep + hh - 2);
-    *h = hh;
+// Product build, the face states of system_flux: e(p), and the interval for
+// eos_sound_at.  a.h = 0 when the EoS is not a table with records (then
+// eos_energy / eos_sound are used).
+__device__ __forceinline__ int eos_energy_h(const DevPhys& P, double rh, double* en, double pr, EosAt& a) {
+  if (P.eqstate == ECHO_EOS_TABLE && P.rec) {
+    if (pr < P.pmin) return 125;
+    if (pr > P.pmax) return 126;
+    eos_at_p(P, pr, a);
+    *en = a.e0 + (pr - a.p0) * a.sl;
     return 0;
   }
-  *h = 0;
+  a.h = 0;
   return eos_energy(P, rh, en, pr);
 }
-// c_s^2(e) for the e just interpolated in bracket h: e lies in the same
-// interval of the e column (e(p) is monotonic; at a node both neighbouring
-// intervals give the node value), so get_sound's search is skipped
-__device__ __forceinline__ double eos_sound_at(const DevPhys& P, int h, double en) {
-  return __ldg(P.tc + h - 2) + (en - __ldg(P.te + h - 2)) * __ldg(P.sl_ce + h - 2);
+// c_s^2(e) for the e just interpolated: e lies in the same interval of the e
+// column (e(p) is monotonic; at a node both neighbouring intervals give the
+// node value), so get_sound's search is skipped
+__device__ __forceinline__ double eos_sound_at(const DevPhys& P, const EosAt& a, double en) {
+  const double2 c = __ldg((const double2*)(P.rec + (a.h - 2)) + 3);
+  return c.x + (en - a.e0) * c.y;
 }
 #endif
 
 // eos_sound: get_sound (eos.f90:590-641) / eos_sound_ana (eos.f90:926-952)
 __device__ __forceinline__ int eos_sound(const DevPhys& P, double rh, double en, double pr, double* cs2) {
   if (P.eqstate == ECHO_EOS_TABLE) {
-    if (en < __ldg(P.te)) return 131;
-    if (en > __ldg(P.te + P.nt - 1)) return 132;
-    int h = SEARCH_E(P, en);
 #ifndef ECHO_EXACT
-    if (P.sl_ce) {
-      *cs2 = __ldg(P.tc + h - 2) + (en - __ldg(P.te + h - 2)) * __ldg(P.sl_ce + h - 2);
+    if (P.rec) {
+      if (en < P.emin) return 131;
+      if (en > P.emax) return 132;
+      EosAt a;
+      eos_at_e(P, en, a);
+      *cs2 = eos_sound_at(P, a, en);
       return 0;
     }
 #endif
+    if (en < __ldg(P.te)) return 131;
+    if (en > __ldg(P.te + P.nt - 1)) return 132;
+    int h = SEARCH_E(P, en);
     double s2 = __ldg(P.tc + h - 1), s1 = __ldg(P.tc + h - 2);
     double e2 = __ldg(P.te + h - 1), e1 = __ldg(P.te + h - 2);
     *cs2 = s1 + (s2 - s1) * (en - e1) / (e2 - e1);
@@ -320,10 +426,35 @@ __device__ __forceinline__ int eos_sound(const DevPhys& P, double rh, double en,
   return 0;
 }
 
+// eos_pressure inside a Newton loop: a is the interval of the last call
+// (a.h = 0 before the first)
+__device__ __forceinline__ int eos_pressure_it(const DevPhys& P, double rh, double en, double* pr, double* dprdrh,
+                                               double* dprden, EosAt& a) {
+#ifndef ECHO_EXACT
+  if (P.eqstate == ECHO_EOS_TABLE && P.rec) return eos_pressure_at(P, en, pr, dprdrh, dprden, a);
+#endif
+  return eos_pressure(P, rh, en, pr, dprdrh, dprden);
+}
+
 // get_derived_data: get_derived_data_tab (eos.f90:645-701) / _ana (eos.f90:956-968)
 __device__ __forceinline__ int get_derived_data(const DevPhys& P, double rh, double pr, double* en,
                                                 double* temp, double* s) {
   if (P.eqstate == ECHO_EOS_TABLE) {
+#ifndef ECHO_EXACT
+    if (P.rec) {
+      if (pr < P.pmin) return 135;
+      if (pr > P.pmax) return 136;
+      EosAt a;
+      eos_at_p(P, pr, a);
+      const double e1 = a.e0, e2 = __ldg(&P.rec[a.h - 2].te1);
+      const double t1 = __ldg(P.tT + a.h - 2), t2 = __ldg(P.tT + a.h - 1);
+      const double fac = (pr - a.p0) / (a.hi - a.p0);
+      *temp = t1 + (t2 - t1) * fac;
+      *en = e1 + (e2 - e1) * fac;
+      *s = (*en + pr) / *temp;
+      return 0;
+    }
+#endif
     if (pr < __ldg(P.tp)) return 135;
     if (pr > __ldg(P.tp + P.nt - 1)) return 136;
     int h = SEARCH_P(P, pr);
@@ -415,31 +546,31 @@ __device__ __forceinline__ double mp5(double f, double f1, double f2, double f3,
 
 // WENO5 one side: f1..f5 in the reference's naming (holib.f90:198-212)
 #ifndef ECHO_EXACT
-// Product build: the scheme in differences of neighbouring values.  With
-// d_i the first and D_i the second differences of a side's stencil f1..f5,
-// 4 (beta_k / 12 + eps) is 13/3 D^2 + t^2 + 4 eps with t = 2 d + D, d + d or
-// D - 2 d; the sub-stencil polynomials are f3 + delta_k with delta_k two terms
-// in d (below, the factor 1/8 and the linear weights 10 and 5 folded into
-// their exactly representable coefficients).  The common denominator of the
-// weights is multiplied through, sum_k d_k delta_k / q_k^2 / sum_k d_k / q_k^2
-// = sum_k d_k delta_k Q_j Q_l / sum_k d_k Q_j Q_l with Q = q^2 (q >= 4e-6, so
-// the products cannot underflow), and the two states share one reciprocal:
-// n1/m1 and n2/m2 = (n1 m2, n2 m1) / (m1 m2), where m1, m2 >= 1e-21 and stay
-// far below 1e150 for the values a run holds.  The difference form needs 56
-// FP64 instructions for both states of a cell (the same in values: 101 for the
-// two states of a face) and rounds less: the cancellations of nearly equal
-// values are the exact differences d_i.
-__device__ __forceinline__ double weno5_q(double D, double t) {  // 4 (beta / 12 + eps)
-  return fma(t, t, fma((13. / 3.) * D, D, 4.e-6));
+// Product build: the scheme in differences of neighbouring values.  With d_i
+// the first and D_i the second differences of a side's stencil f1..f5:
+//  - 4 (beta_k / 12 + eps) is 4 d^2 + 4 d D + 16/3 D^2 + 4 eps with the d
+//    beside f3 and the sub-stencil's D (4 d^2 - 4 d D for the third);
+//  - the sub-stencil values are f3 + d / 2 + 3/8 D1, f3 + d / 2 + 3/8 D2 and
+//    f3 + d / 2 + 1/2 D2 - 1/8 D3, so a state is f3 + d / 2 plus a weighted
+//    mean of second differences;
+//  - the common denominator of the weights is multiplied through,
+//    sum_k d_k x_k / q_k^2 / sum_k d_k / q_k^2 = sum_k d_k x_k Q_j Q_l /
+//    sum_k d_k Q_j Q_l with Q = q^2 (q >= 4e-6, so the products cannot
+//    underflow), and the two states share one reciprocal: n1/m1 and n2/m2 =
+//    (n1 m2, n2 m1) / (m1 m2), where m1, m2 >= 1e-21 and stay far below 1e150
+//    for the values a run holds.
+// 50 FP64 instructions for both states of a cell (written in values, 101 for
+// the two states of a face), with less rounding: the cancellations of nearly
+// equal values are the exact differences.
+__device__ __forceinline__ double weno5_q(double D, double d4, double A) {  // d4 = 4 d, A = 4 d^2 + 4 eps
+  return fma(D, fma(16. / 3., D, d4), A);
 }
-// numerator (without f3) and denominator of a side from its first differences
-// and the products w1 = Q2 Q3, w2 = Q1 Q3, w3 = Q1 Q2
-__device__ __forceinline__ void weno5_nm(double d0, double d1, double d2, double d3, double w1, double w2, double w3,
+// 8/3 of the numerator beyond f3 + d / 2, and the denominator, of a side from
+// its second differences and w1 = Q2 Q3, w2 = Q1 Q3, w3 = Q1 Q2; g = w2 D2,
+// H = 20/3 D2
+__device__ __forceinline__ void weno5_nm(double D1, double D3, double g, double H, double w1, double w2, double w3,
                                          double& n, double& m) {
-  const double e1 = fma(0.875, d1, -0.375 * d0);   // (7 d1 - 3 d0) / 8
-  const double e2 = fma(3.75, d2, 1.25 * d1);      // 10 (3 d2 + d1) / 8
-  const double e3 = fma(3.125, d2, -0.625 * d3);   // 5 (5 d2 - d3) / 8
-  n = fma(w3, e3, fma(w2, e2, w1 * e1));
+  n = fma(w3, fma(-5. / 3., D3, H), fma(10., g, w1 * D1));
   m = fma(5., w3, fma(10., w2, w1));
 }
 // Both face states of one cell from its five-point stencil f1..f5 =
@@ -451,33 +582,69 @@ __device__ __forceinline__ void weno5_cell(double f1, double f2, double f3, doub
                                            double& minus) {
   const double d0 = f2 - f1, d1 = f3 - f2, d2 = f4 - f3, d3 = f5 - f4;
   const double Da = d1 - d0, Db = d2 - d1, Dc = d3 - d2;
-  const double qa = weno5_q(Da, fma(2., d1, Da)), qb = weno5_q(Db, d1 + d2), qc = weno5_q(Dc, fma(-2., d2, Dc));
+  const double e1 = 4. * d1, e2 = -4. * d2;
+  const double A1 = fma(e1, d1, 4.e-6), A2 = fma(-e2, d2, 4.e-6);
+  const double qa = weno5_q(Da, e1, A1), qb = weno5_q(Db, e1, A1), qc = weno5_q(Dc, e2, A2);
   const double Qa = qa * qa, Qb = qb * qb, Qc = qc * qc;
   const double wbc = Qb * Qc, wac = Qa * Qc, wab = Qa * Qb;
+  const double g = wac * Db, H = (20. / 3.) * Db;
   double np, mp, nm, mm;
-  weno5_nm(d0, d1, d2, d3, wbc, wac, wab, np, mp);
-  weno5_nm(d3, d2, d1, d0, wab, wac, wbc, nm, mm);  // reversed: the differences change sign
-  const double inv = rcp_h3(mp * mm);
-  plus = fma(np * mm, inv, f3);
-  minus = fma(-nm * mp, inv, f3);
+  weno5_nm(Da, Dc, g, H, wbc, wac, wab, np, mp);
+  weno5_nm(Dc, Da, g, H, wab, wac, wbc, nm, mm);  // reversed: the first differences change sign
+  const double inv = 0.375 * rcp_h3(mp * mm);
+  plus = f3 + fma(np * mm, inv, 0.5 * d1);  // one rounding at the size of f3
+  minus = f3 + fma(nm * mp, inv, -0.5 * d2);
+}
+// weno5_cell of the two neighbouring cells f[2] and f[3]: they share three first
+// and two second differences and a smoothness term (42.5 FP64 instructions a
+// cell)
+__device__ __forceinline__ void weno5_pair(const double f[6], double plus[2], double minus[2]) {
+  double d[5], D[5], e[4], A[4];
+#pragma unroll
+  for (int i = 0; i < 5; i++) d[i] = f[i + 1] - f[i];
+#pragma unroll
+  for (int i = 1; i < 5; i++) D[i] = d[i] - d[i - 1];
+#pragma unroll
+  for (int i = 1; i < 4; i++) {
+    e[i] = 4. * d[i];
+    A[i] = fma(e[i], d[i], 4.e-6);
+  }
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const double Da = D[c + 1], Db = D[c + 2], Dc = D[c + 3];
+    const double qa = weno5_q(Da, e[c + 1], A[c + 1]), qb = weno5_q(Db, e[c + 1], A[c + 1]);
+    const double qc = weno5_q(Dc, -e[c + 2], A[c + 2]);
+    const double Qa = qa * qa, Qb = qb * qb, Qc = qc * qc;
+    const double wbc = Qb * Qc, wac = Qa * Qc, wab = Qa * Qb;
+    const double g = wac * Db, H = (20. / 3.) * Db;
+    double np, mp, nm, mm;
+    weno5_nm(Da, Dc, g, H, wbc, wac, wab, np, mp);
+    weno5_nm(Dc, Da, g, H, wab, wac, wbc, nm, mm);
+    const double inv = 0.375 * rcp_h3(mp * mm);
+    plus[c] = f[c + 2] + fma(np * mm, inv, 0.5 * d[c + 1]);
+    minus[c] = f[c + 2] + fma(nm * mp, inv, -0.5 * d[c + 2]);
+  }
 }
 // Left and right state of the face between s[2] and s[3]
 __device__ __forceinline__ void weno5_face(const double s[6], double& gl, double& gr) {
   const double d0 = s[1] - s[0], d1 = s[2] - s[1], d2 = s[3] - s[2], d3 = s[4] - s[3], d4 = s[5] - s[4];
   const double D1 = d1 - d0, D2 = d2 - d1, D3 = d3 - d2, D4 = d4 - d3;
-  double q1 = weno5_q(D1, fma(2., d1, D1)), q2 = weno5_q(D2, d1 + d2), q3 = weno5_q(D3, fma(-2., d2, D3));
-  double Q1 = q1 * q1, Q2 = q2 * q2, Q3 = q3 * q3, nl, ml, nr, mr;
-  weno5_nm(d0, d1, d2, d3, Q2 * Q3, Q1 * Q3, Q1 * Q2, nl, ml);
-  q1 = weno5_q(D4, fma(-2., d3, D4));
-  q2 = weno5_q(D3, d2 + d3);
-  q3 = weno5_q(D2, fma(2., d2, D2));
+  const double e1 = 4. * d1, e2 = 4. * d2, e3 = 4. * d3;
+  const double A1 = fma(e1, d1, 4.e-6), A2 = fma(e2, d2, 4.e-6), A3 = fma(e3, d3, 4.e-6);
+  double q1 = weno5_q(D1, e1, A1), q2 = weno5_q(D2, e1, A1), q3 = weno5_q(D3, -e2, A2);
+  double Q1 = q1 * q1, Q2 = q2 * q2, Q3 = q3 * q3, w = Q1 * Q3, nl, ml, nr, mr;
+  weno5_nm(D1, D3, w * D2, (20. / 3.) * D2, Q2 * Q3, w, Q1 * Q2, nl, ml);
+  q1 = weno5_q(D4, -e3, A3);
+  q2 = weno5_q(D3, -e3, A3);
+  q3 = weno5_q(D2, e2, A2);
   Q1 = q1 * q1;
   Q2 = q2 * q2;
   Q3 = q3 * q3;
-  weno5_nm(d4, d3, d2, d1, Q2 * Q3, Q1 * Q3, Q1 * Q2, nr, mr);
-  const double inv = rcp_h3(ml * mr);
-  gl = fma(nl * mr, inv, s[2]);
-  gr = fma(-nr * ml, inv, s[3]);
+  w = Q1 * Q3;
+  weno5_nm(D4, D2, w * D3, (20. / 3.) * D3, Q2 * Q3, w, Q1 * Q2, nr, mr);
+  const double inv = 0.375 * rcp_h3(ml * mr);
+  gl = s[2] + fma(nl * mr, inv, 0.5 * d1);
+  gr = s[3] + fma(nr * ml, inv, -0.5 * d3);
 }
 #else
 __device__ __forceinline__ double weno5_side(double f1, double f2, double f3, double f4, double f5) {
@@ -643,6 +810,19 @@ __device__ __forceinline__ void recon_cell(int recal, const double f[5], double&
       break;
     }
   }
+}
+
+// recon_cell of the N neighbouring cells f[2], f[3], ... from f[0..N+3]
+template <int REC, int N>
+__device__ __forceinline__ void recon_cells(int recal, const double* f, double* plus, double* minus) {
+#ifndef ECHO_EXACT
+  if (REC == ECHO_REC_WENO5 && N == 2) {
+    weno5_pair(f, plus, minus);
+    return;
+  }
+#endif
+#pragma unroll
+  for (int i = 0; i < N; i++) recon_cell<REC>(recal, f + i, plus[i], minus[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -838,8 +1018,8 @@ __device__ __forceinline__ int system_flux(const DevPhys& P, const Metric& M, do
 #ifdef ECHO_EXACT
   int err = eos_energy(P, rh, &en, pr);
 #else
-  int hb = 0;
-  int err = eos_energy_h(P, rh, &en, pr, &hb);
+  EosAt at;
+  int err = eos_energy_h(P, rh, &en, pr, at);
 #endif
   if (err) return err;
   double v2 = g1 * vx * vx + g2 * vy * vy + g3 * vz * vz;
@@ -1015,8 +1195,8 @@ __device__ __forceinline__ int system_flux(const DevPhys& P, const Metric& M, do
 #ifdef ECHO_EXACT
   err = eos_sound(P, rh, en, pr, &cs2);
 #else
-  if (hb)
-    cs2 = eos_sound_at(P, hb, en);
+  if (at.h)
+    cs2 = eos_sound_at(P, at, en);
   else
     err = eos_sound(P, rh, en, pr, &cs2);
 #endif

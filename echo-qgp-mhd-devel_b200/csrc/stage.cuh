@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(ECHO_STAGE_NT, ECHO_STAGE_MINB) stage_kernel(S
       }
       // 5. sources, RK combination (or the stage right-hand side), con2prim
       const size_t c = (size_t)k * nxy + (size_t)gy * g.nx + gx;
-      update_finish<KIND, SEED, IMEX>(U, own ? c : 0, own, gx, gy, k, du, dv);
+      update_finish<KIND, SEED, IMEX, C2P_ANY>(U, own ? c : 0, own, gx, gy, k, du, dv);
     }
   }
   block_max_atomic(am[0], &U.sc->amax_bits[0], red);

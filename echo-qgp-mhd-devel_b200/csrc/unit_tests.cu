@@ -172,6 +172,7 @@ extern "C" int echo_gpu_test_c2p(const EchoParams* p, const double* eos_table, i
   M.g3 = g3;
   M.gp = gp;
   M.gm = 1. / gp;
+  M.ig3 = 1. / g3;
   M.t = gp;
   M.t3 = pow(gp, 3.);
   switch (kind) {
@@ -280,6 +281,7 @@ extern "C" int echo_gpu_test_c2p_seeded(const EchoParams* p, const double* eos_t
   M.g3 = g3;
   M.gp = gp;
   M.gm = 1. / gp;
+  M.ig3 = 1. / g3;
   M.t = gp;
   M.t3 = pow(gp, 3.);
   unsigned blocks = (unsigned)((ncells + 127) / 128);
