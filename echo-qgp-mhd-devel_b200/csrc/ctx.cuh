@@ -67,6 +67,7 @@ struct EchoCtx {
   cudaStream_t copy_stream;
   cudaEvent_t ev_u, ev_u_fork;
   int wait_u;
+  int snap;  // the first stage's update takes the viscous vnewstep (snapshot_vnewstep)
   // the fused stage kernel (stage.cuh): usable, on, tile, segment, launch
   int st_ok, st_on, st_tx, st_ty, st_zseg, st_nt;
   unsigned st_grid;
@@ -101,12 +102,12 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
 namespace echo {
 
 template <int KIND>
-void launch_faces(EchoCtx* c, int mask);
+void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last = nullptr);
 template <int KIND>
 void launch_update(EchoCtx* c, int irk, int mode, double* du_out);
-// what: 1 = repair only, 2 = smoothing only, 3 = both
+// what: 1 = repair only, 2 = smoothing only, 3 = both; then: RepairArgs::then
 template <int KIND>
-void launch_repair_smooth(EchoCtx* c, int what = 3);
+void launch_repair_smooth(EchoCtx* c, int what, int then);
 template <int KIND>
 void launch_p2c(EchoCtx* c);
 template <int KIND>

@@ -205,7 +205,7 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
     }                                                             \
   } while (0)
 
-static void launch_scalars(EchoCtx* c, int irk, int mode = 0) {
+static ScalarArgs scalar_args(const EchoCtx* c, int irk, int mode, int reset) {
   ScalarArgs S;
   S.sc = c->d_sc;
   S.g = c->g;
@@ -216,62 +216,65 @@ static void launch_scalars(EchoCtx* c, int irk, int mode = 0) {
   S.nrk = c->p.nrk;
   S.divclean = c->p.divclean;
   S.mode = mode;
-  stage_scalars_kernel<<<1, 1, 0, c->stream>>>(S);
+  S.reset = reset;
+  return S;
+}
+static void launch_scalars(EchoCtx* c, int irk, int mode = 0, int reset = 0) {
+  stage_scalars_kernel<<<1, 1, 0, c->stream>>>(scalar_args(c, irk, mode, reset));
 }
 
-// The flux sweeps of a stage: one launch for all directions, or, with
-// par_sweeps off and for per-kernel profiling, one for each in order.
-static void launch_sweeps(EchoCtx* c) {
+// The flux sweeps of a stage and, S given, its scalar logic: one launch, or,
+// with par_sweeps off and for per-kernel profiling, one for each in order.
+static void launch_sweeps(EchoCtx* c, const ScalarArgs* S = nullptr) {
   int mask = 0;
   for (int d = 0; d < 3; d++)
     if ((d == 0 ? c->g.nx : d == 1 ? c->g.ny : c->g.nz) > 1) mask |= 1 << d;
-  if (!mask) return;
-  if (c->par_sweeps && !c->marks) {
-    DISPATCH(c, launch_faces, c, mask);
+  if (mask && c->par_sweeps && !c->marks) {
+    DISPATCH(c, launch_faces, c, mask, S);
     return;
   }
   for (int d = 0; d < 3; d++)
     if (mask >> d & 1) {
-      DISPATCH(c, launch_faces, c, 1 << d);
+      DISPATCH(c, launch_faces, c, 1 << d, nullptr);
       mark(c, PK_FACES_X + d);
     }
-}
-
-// the flux sweeps of a stage; the CFL maxima start from zero
-static void enqueue_sweeps(EchoCtx* c) {
-  cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream);
-  launch_sweeps(c);
+  if (S) {
+    stage_scalars_kernel<<<1, 1, 0, c->stream>>>(*S);
+    mark(c, PK_SCALARS);
+  }
 }
 
 // IMEX-SSP3(4,3,3) stage (evolve.f90:204-267), all asynchronous
-static void enqueue_stage_ssp(EchoCtx* c, int irk) {
+static void enqueue_stage_ssp(EchoCtx* c, int irk, int then) {
+  const bool fused = c->st_ok && c->st_on;
   if (irk == 1) {
     launch_scalars(c, 1, 1);  // dt from the previous stage's speeds
   } else {
     if (irk == 2) c->ucur = 1 - c->ucur;  // U[ucur] becomes the u built from u0 = U[1-ucur]
-    cudaMemsetAsync(&c->d_sc->nfail, 0, sizeof(int), c->stream);
-    cudaMemsetAsync(&c->d_sc->c2p_iters, 0, sizeof(unsigned long long), c->stream);
     DISPATCH(c, launch_ssp_combine, c, irk);
     mark(c, PK_UPDATE);
     // smoothing at the end of these stages would act only on values the next
     // combination overwrites, so the reference's smoothing survives only
     // after the final combination
-    DISPATCH(c, launch_repair_smooth, c, 1);
+    DISPATCH(c, launch_repair_smooth, c, 1, 0);
     mark(c, PK_REPAIR);
     c->vcur = 1 - c->vcur;
   }
-  if (c->st_ok && c->st_on) {
+  // the CFL maxima start from zero; the counters of the combination that
+  // follows the stage too (the stage-4 solve and the final combination share
+  // one count of con2prim iterations)
+  cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream);
+  const int reset = irk < 4 ? 3 : 1;
+  if (fused) {
     // sweeps + right-hand side in one kernel; the GLM scalars after it (the
     // right-hand side reads none of them)
-    cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream);
     DISPATCH(c, launch_stage, c, irk, MODE_RHS, c->d_dussp[irk - 1]);
     mark(c, PK_STAGE);
-    launch_scalars(c, irk, 2);
+    launch_scalars(c, irk, 2, reset);
     mark(c, PK_SCALARS);
   } else {
-    enqueue_sweeps(c);
-    launch_scalars(c, irk, 2);
-    mark(c, PK_SCALARS);
+    const ScalarArgs S = scalar_args(c, irk, 2, reset);
+    launch_sweeps(c, &S);
     DISPATCH(c, launch_update, c, irk, MODE_RHS, c->d_dussp[irk - 1]);
     mark(c, PK_UPDATE);
   }
@@ -280,60 +283,60 @@ static void enqueue_stage_ssp(EchoCtx* c, int irk) {
     mark(c, PK_UPDATE);
   }
   if (irk == 4) {
-    cudaMemsetAsync(&c->d_sc->nfail, 0, sizeof(int), c->stream);
     DISPATCH(c, launch_ssp_combine, c, 5);
     mark(c, PK_UPDATE);
-    DISPATCH(c, launch_repair_smooth, c, 3);
+    DISPATCH(c, launch_repair_smooth, c, 3, then);
     mark(c, PK_REPAIR);
     c->vcur = 1 - c->vcur;
   }
 }
 
-// one explicit RK stage, all asynchronous
 // the stream waits for the host copy of u of echo_gpu_advance_host
 static void join_u(EchoCtx* c) {
   cudaStreamWaitEvent(c->stream, c->ev_u, 0);
   c->wait_u = 0;
 }
 
-static void enqueue_stage(EchoCtx* c, int irk) {
+// whether stage irk of this run is one fused launch: it needs dt before the
+// faces, so every stage but the first, and the first with divergence cleaning
+// (dt = CFL, evolve.f90:734-735)
+static bool stage_is_fused(const EchoCtx* c, int irk) { return c->st_ok && c->st_on && (irk > 1 || c->p.divclean); }
+
+// One stage, all asynchronous.  then: what the repair's launch does after it
+// (RepairArgs::then) beside resetting the CFL maxima of an explicit stage,
+// which are zero between stages.
+static void enqueue_stage(EchoCtx* c, int irk, int then = 0) {
   if (c->p.nrk == ECHO_SSP) {
-    enqueue_stage_ssp(c, irk);
+    enqueue_stage_ssp(c, irk, then);
     return;
   }
-  cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream);
-  // the fused stage needs dt before the faces: every stage but the first,
-  // and the first with divergence cleaning (dt = CFL, evolve.f90:734-735)
-  if (c->st_ok && c->st_on && (irk > 1 || c->p.divclean)) {
-    launch_scalars(c, irk, 3);
-    cudaMemsetAsync(&c->d_sc->nfail, 0, sizeof(int), c->stream);
-    cudaMemsetAsync(&c->d_sc->c2p_iters, 0, sizeof(unsigned long long), c->stream);
+  if (stage_is_fused(c, irk)) {
+    launch_scalars(c, irk, 3, 3);
     mark(c, PK_SCALARS);
     DISPATCH(c, launch_stage, c, irk, MODE_RK, (double*)nullptr);
     mark(c, PK_STAGE);
     launch_scalars(c, irk, 4);
     mark(c, PK_SCALARS);
   } else {
-    launch_sweeps(c);
+    const ScalarArgs S = scalar_args(c, irk, 0, 3);
+    launch_sweeps(c, &S);
     if (c->wait_u) join_u(c);  // the update reads u
-    launch_scalars(c, irk);
-    cudaMemsetAsync(&c->d_sc->nfail, 0, sizeof(int), c->stream);
-    cudaMemsetAsync(&c->d_sc->c2p_iters, 0, sizeof(unsigned long long), c->stream);
-    mark(c, PK_SCALARS);
     DISPATCH(c, launch_update, c, irk, MODE_RK, (double*)nullptr);
     mark(c, PK_UPDATE);
   }
   // stage 1 wrote the new u into the other buffer: it becomes current before
   // the repair and the smoothing, which act on the new u
   if (irk == 1) c->ucur = 1 - c->ucur;
-  DISPATCH(c, launch_repair_smooth, c, 3);
+  DISPATCH(c, launch_repair_smooth, c, 3, then | 1);
   mark(c, PK_REPAIR);
   c->vcur = 1 - c->vcur;
 }
 
 static void snapshot_vnewstep(EchoCtx* c) {
-  // vnewstep = v (echo.f90:193-201); only the viscous time derivatives read it
-  if (c->p.viscosity)
+  // vnewstep = v (echo.f90:193-201); only the viscous time derivatives read
+  // it.  The first explicit stage's update takes it cell by cell.
+  c->snap = c->p.viscosity && c->p.nrk != ECHO_SSP && !stage_is_fused(c, 1);
+  if (c->p.viscosity && !c->snap)
     cudaMemcpyAsync(c->d_vh[c->vn], c->d_v[c->vcur], sizeof(double) * c->g.ncell * 4, cudaMemcpyDeviceToDevice,
                     c->stream);
   if (c->keep_old) {  // the full vnewstep / unewstep of the reference, for dump.dat
@@ -343,9 +346,10 @@ static void snapshot_vnewstep(EchoCtx* c) {
   }
 }
 
-// end of step: vold = vnewstep, uold = unewstep (echo.f90:240-241) are role swaps
-static void end_step(EchoCtx* c) {
-  end_step_kernel<<<1, 1, 0, c->stream>>>(c->d_sc, c->p.coordinates);
+// end of step: vold = vnewstep, uold = unewstep (echo.f90:240-241) are role
+// swaps; the scalars are the last repair's (done) or a launch of their own
+static void end_step(EchoCtx* c, bool done = false) {
+  if (!done) end_step_kernel<<<1, 1, 0, c->stream>>>(c->d_sc, c->p.coordinates);
   mark(c, PK_END);
   if (c->p.viscosity) c->vn = 1 - c->vn;
   if (c->keep_old) c->on = 1 - c->on;
@@ -357,8 +361,10 @@ static void enqueue_step(EchoCtx* c) {
   // other paths touch u at once
   if (c->wait_u && (c->keep_old || c->p.nrk == ECHO_SSP || (c->st_ok && c->st_on))) join_u(c);
   snapshot_vnewstep(c);
-  for (int irk = 1; irk <= c->p.nrk; irk++) enqueue_stage(c, irk);
-  end_step(c);
+  // the smoothing after the last repair still reads the step's time
+  const bool end = !(c->p.viscosity && c->p.enable_smooth_viscosity) && !c->marks;
+  for (int irk = 1; irk <= c->p.nrk; irk++) enqueue_stage(c, irk, end && irk == c->p.nrk ? 2 : 0);
+  end_step(c, end);
   if (c->wait_u) join_u(c);
 }
 
@@ -802,6 +808,8 @@ int echo_gpu_restart(EchoCtx* c, const void* blob) {
   size_t nvc = (size_t)c->nv * c->g.ncell;
   const char* p = (const char*)blob + sizeof(h);
   c->vcur = c->ucur = c->vn = c->on = 0;
+  if (c->p.nrk != ECHO_SSP) memset(h.sc.amax_bits, 0, sizeof(h.sc.amax_bits));  // zero between explicit stages
+  h.sc.done = 0;
   CK(cudaMemcpyAsync(c->d_sc, &h.sc, sizeof(DevScalars), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->d_v[0], p, sizeof(double) * nvc, cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->d_u[0], p + sizeof(double) * nvc, sizeof(double) * nvc, cudaMemcpyHostToDevice,
@@ -1083,6 +1091,8 @@ int echo_gpu_rhs(EchoCtx* c, double* du, double* amax3) {
   if (du) CK(cudaMemcpyAsync(du, c->d_du, sizeof(double) * nvc, cudaMemcpyDeviceToHost, c->stream));
   int r = read_scalars(c);
   if (r) return r;
+  // an IMEX-SSP step starts from the maxima of the last sweeps
+  if (c->p.nrk != ECHO_SSP) CK(cudaMemsetAsync(c->d_sc->amax_bits, 0, sizeof(unsigned long long) * 3, c->stream));
   if (amax3)
     for (int d = 0; d < 3; d++) {
       unsigned long long b = c->h_sc->amax_bits[d];

@@ -38,6 +38,10 @@ struct SweepArgs {
   FaceArgs A[3];          // x, y, eta
   unsigned first[4];      // block range of each direction
   int lw;                 // log2 of the pencils of a y or eta tile
+  // with last set, the block that finishes last runs the stage's scalar logic:
+  // one launch fewer on the chain of every stage
+  int last;
+  ScalarArgs S;
 };
 
 // 64 KB of shared memory a block at most: 2 x (NV + 4) x 256 doubles
@@ -584,7 +588,17 @@ __global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC))
     dir = 2;
     amax = face_tile<KIND, 2, REC, LC, CPT, NG>(S.A[2], b - S.first[2], S.lw, sm);
   }
-  block_max_atomic(amax, &S.A[0].sc->amax_bits[dir], red);
+  DevScalars* sc = S.A[0].sc;
+  block_max_atomic(amax, &sc->amax_bits[dir], red);
+  // thread 0 has the block's maximum and, past the barrier above, every
+  // thread's aflux behind it
+  if (S.last && threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&sc->done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      stage_scalars_last(S.S);
+    }
+  }
 }
 
 }  // namespace echo

@@ -27,7 +27,8 @@ struct DevScalars {
   double glm_ch, glm_ch_old, aflux[3], expfact;
   unsigned long long amax_bits[3];
   unsigned long long err_key;  // (cell << 20) | code, min over failures
-  int nfail, pad;
+  int nfail;
+  unsigned done;               // blocks of the running sweep that have finished; 0 between sweeps
   unsigned long long c2p_iters, c2p_cells, repairs, fallbacks;
   unsigned long long check_bits;  // check_temp maximum (bit pattern of a double >= 0)
   unsigned long long brackets;    // con2prim solves that fell back to the bracketed BRENTM
@@ -475,12 +476,6 @@ __device__ __forceinline__ void block_max_atomic(double m, unsigned long long* d
   }
 }
 
-}  // namespace echo
-
-#include "faces.cuh"
-
-namespace echo {
-
 // ---------------------------------------------------------------------------
 // scalar logic of evolve_main (evolve.f90:156-201) and evolve_dt (:723-764)
 // ---------------------------------------------------------------------------
@@ -489,6 +484,7 @@ struct ScalarArgs {
   Grid g;
   double cfl, maxdt, glm_alpha;
   int irk, nrk, divclean;
+  int reset;  // the counters that start from zero: 1 nfail, 2 c2p_iters
   int mode;  // 0: explicit RK stage (after the sweeps); 1: IMEX-SSP dt (before the
              // sweeps of stage 1, from the previous stage's speeds); 2: IMEX-SSP GLM;
              // 3, 4: the fused stage kernel's halves of mode 0 -- 3 before it
@@ -553,7 +549,41 @@ __device__ __forceinline__ void stage_scalars(const ScalarArgs& A) {
   if (A.divclean && A.mode != 1) sc->expfact = exp(-sc->glm_ch * sc->glm_ch * A.glm_alpha * (sc->dt / 2.));
 }
 
-static __global__ void stage_scalars_kernel(ScalarArgs A) { stage_scalars(A); }
+__device__ __forceinline__ void reset_counters(DevScalars* sc, int reset) {
+  if (reset & 1) sc->nfail = 0;
+  if (reset & 2) sc->c2p_iters = 0;
+}
+static __global__ void stage_scalars_kernel(ScalarArgs A) {
+  stage_scalars(A);
+  reset_counters(A.sc, A.reset);
+}
+
+// The same by the last block of a sweep (one thread): the run's scalars are
+// read past the L1, where lines from before the other blocks' atomics may
+// still be.
+static __device__ __noinline__ void stage_scalars_last(const ScalarArgs& A) {
+  union {
+    DevScalars s;
+    unsigned long long w[sizeof(DevScalars) / 8];
+  } u;
+  static_assert(sizeof(DevScalars) % 8 == 0, "copied in words of 8 bytes");
+  for (unsigned i = 0; i < sizeof(DevScalars) / 8; i++) u.w[i] = __ldcg((const unsigned long long*)A.sc + i);
+  ScalarArgs B = A;
+  B.sc = &u.s;
+  stage_scalars(B);
+  A.sc->glm_ch = u.s.glm_ch;
+  A.sc->glm_ch_old = u.s.glm_ch_old;
+  A.sc->dt = u.s.dt;
+  A.sc->expfact = u.s.expfact;
+  reset_counters(A.sc, A.reset);
+  A.sc->done = 0;
+}
+
+}  // namespace echo
+
+#include "faces.cuh"
+
+namespace echo {
 
 // end of step (echo.f90:211-241)
 __device__ __forceinline__ void end_step_scalars(DevScalars* sc, int coordinates) {
@@ -1112,6 +1142,9 @@ struct RepairArgs {
   int coordinates, algo;
   double maxspeed, tol;
   double h_alpha;  // resistive implicit stages: a_ii, the solve uses h = a_ii dt
+  // after the repair, by one thread: 1 the CFL maxima start from zero again
+  // (explicit stages), 2 the end of the step (end_step_scalars)
+  int then;
 };
 
 template <int KIND>
@@ -1317,10 +1350,17 @@ __device__ __forceinline__ void repair_grid(const RepairArgs& A, int& s_any, int
 
 template <int KIND>
 __global__ void __launch_bounds__(256) repair_kernel(RepairArgs A) {
-  if (A.sc->nfail == 0) return;
-  __shared__ int s_any, s_stop;
-  __shared__ unsigned s_list[ECHO_REPAIR_LIST];
-  repair_grid<KIND, ECHO_REPAIR_LIST>(A, s_any, s_stop, s_list);
+  if (A.sc->nfail != 0) {
+    __shared__ int s_any, s_stop;
+    __shared__ unsigned s_list[ECHO_REPAIR_LIST];
+    repair_grid<KIND, ECHO_REPAIR_LIST>(A, s_any, s_stop, s_list);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    if (A.then & 1)
+      for (int d = 0; d < 3; d++) A.sc->amax_bits[d] = 0;
+    if (A.then & 2) end_step_scalars(A.sc, A.coordinates);
+  }
 }
 
 // evolve_smooth_viscosity (evolve.f90:1159-1207)

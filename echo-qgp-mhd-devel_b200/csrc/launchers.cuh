@@ -21,11 +21,16 @@ inline int sweep_lc(const EchoCtx* c, int mask) {
   return t >= 2 * 148 ? 8 : 5;
 }
 
-// the sweeps of the directions in mask (bit d: direction d), one launch
+// the sweeps of the directions in mask (bit d: direction d), one launch; last,
+// if given: the stage's scalar logic by the block that finishes last
 template <int KIND>
-void launch_faces(EchoCtx* c, int mask) {
+void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last) {
   SweepArgs S;
   memset(&S, 0, sizeof(S));
+  if (last) {
+    S.last = 1;
+    S.S = *last;
+  }
   // pencils of a tile of the y and eta sweeps: 16, or as many as leave
   // face_mode cells of each in a tile (echo_gpu_set_faces)
   const int lc = sweep_lc(c, mask);
@@ -105,7 +110,7 @@ void launch_update(EchoCtx* c, int irk, int mode, double* du_out) {
   }
   A.mlp.frag = c->d_mlp_frag;
   A.mlp.par = c->d_mlp_par;
-  A.vsnap = nullptr;
+  A.vsnap = Traits<KIND>::VISC && c->snap && irk == 1 && mode == MODE_RK ? c->d_vh[c->vn] : nullptr;
   if (A.algo == ECHO_C2P_MLP && !c->d_mlp_frag) A.algo = ECHO_C2P_NEWTON;  // no network loaded
   unsigned blocks = (unsigned)((c->g.ncell + 127) / 128);
   // the learned seed: RMHD (ideal, resistive) and viscous runs
@@ -289,8 +294,9 @@ void launch_stage(EchoCtx* c, int irk, int mode, double* du_out) {
 }
 
 template <int KIND>
-void launch_repair_smooth(EchoCtx* c, int what) {
+void launch_repair_smooth(EchoCtx* c, int what, int then) {
   RepairArgs R;
+  R.then = then;
   R.P = c->P;
   R.g = c->g;
   R.vold = c->d_v[c->vcur];
@@ -668,11 +674,11 @@ void batch_occupancy(const EchoBatch* b, int* per_sm) {
 }  // namespace echo
 
 #define ECHO_INSTANTIATE_GRID(K)                                              \
-  template void echo::launch_faces<K>(EchoCtx*, int);                         \
+  template void echo::launch_faces<K>(EchoCtx*, int, const ScalarArgs*);                         \
   template int echo::setup_stage<K>(EchoCtx*, int, int, int);                 \
   template void echo::launch_stage<K>(EchoCtx*, int, int, double*);           \
   template void echo::launch_update<K>(EchoCtx*, int, int, double*);          \
-  template void echo::launch_repair_smooth<K>(EchoCtx*, int);                 \
+  template void echo::launch_repair_smooth<K>(EchoCtx*, int, int);                 \
   template void echo::launch_p2c<K>(EchoCtx*);                                \
   template void echo::launch_ssp_combine<K>(EchoCtx*, int);                   \
   template void echo::launch_ssp_stage1<K>(EchoCtx*);
