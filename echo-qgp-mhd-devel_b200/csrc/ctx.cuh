@@ -102,7 +102,7 @@ int echo_setup_phys(const EchoParams* p, const double* eos_table, int n_eos, Dev
 namespace echo {
 
 template <int KIND>
-void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last = nullptr);
+void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last = nullptr, bool check = false);
 template <int KIND>
 void launch_update(EchoCtx* c, int irk, int mode, double* du_out);
 // what: 1 = repair only, 2 = smoothing only, 3 = both; then: RepairArgs::then

@@ -382,11 +382,45 @@ __device__ __forceinline__ void face_one(const FaceArgs& A, const Metric& M, uns
   }
 }
 
+// The checks of a face alone (face_one without its flux): the EoS range and
+// superluminal errors of both states, left first, and the signal speed, which
+// is the light cone's.  Resistive runs, first IMEX-SSP stage: the flux of U1
+// has weight 0 in every later combination, its errors and the speed of the
+// cleaning wave are all that stage leaves behind.
+template <int KIND, int DIR, int C>
+__device__ __forceinline__ void face_check(const FaceArgs& A, const Metric& M, unsigned base, unsigned stride, int n,
+                                           int c, int ta, int tb, double* wl, double* wr, double& amax) {
+  const Grid& g = A.g;
+  auto speed2 = [&](const double* w) {
+    return w[KVX * C] * w[KVX * C] + w[KVY * C] * w[KVY * C] + M.g3 * (w[KVZ * C] * w[KVZ * C]);
+  };
+  if (wl[KPR * C] <= 0 || wr[KPR * C] <= 0 || speed2(wl) >= 1. || speed2(wr) >= 1.)
+    fix_states<KIND>(A, M, base, stride, n, c, wl, wr, C);
+  auto bad = [&](const double* w) {
+    if (A.P.eqstate == ECHO_EOS_TABLE) {  // eos_energy
+      if (w[KPR * C] < __ldg(A.P.tp)) return 125;
+      if (w[KPR * C] > __ldg(A.P.tp + A.P.nt - 1)) return 126;
+    }
+    return speed2(w) > 1. ? 333 : 0;
+  };
+  int err = bad(wl);
+  if (!err) err = bad(wr);
+  amax = 0.;
+  if (err) {
+    const size_t cell = base + (size_t)((c >= 1 ? c : 1) - 1) * stride;
+    atomicMin(&A.sc->err_key, ((unsigned long long)cell << 20) | (unsigned long long)err);
+    return;
+  }
+  amax = 1. / sqrt(DIR == 2 ? M.g3 : 1.);
+  const int na = DIR == 0 ? g.ny : g.nx, nb = DIR == 2 ? g.ny : g.nz;
+  if (c == n && ta == na - 1 && tb == nb - 1) A.sc->aflux[DIR] = amax;
+}
+
 // One tile of the sweep along DIR; returns the largest signal speed of this
 // thread's faces.  Called by every thread of the block: NG groups of C / CPT
 // threads, the groups sharing the variables of phase 1.  sm:
-// tile_smem<KIND>(LC) bytes.
-template <int KIND, int DIR, int REC, int LC, int CPT, int NG>
+// tile_smem<KIND>(LC) bytes.  CHECK: velocity and pressure, face_check.
+template <int KIND, int DIR, int REC, int LC, int CPT, int NG, bool CHECK>
 __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, int lw, double* sm) {
   typedef Traits<KIND> T;
   constexpr int NV = T::NV, C = 1 << LC, NT = C / CPT, NS = CPT + 4, UNROLL = ECHO_SWEEP_UNROLL;
@@ -474,8 +508,8 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
       }
     };
     // pi^{eta eta} of a face state follows from the others (derived_pi_zz)
-    const int nr = T::VISC && A.P.obtained_zz ? NV - 1 : NV;
-    int k = grp;
+    const int nr = CHECK ? KPR + 1 : T::VISC && A.P.obtained_zz ? NV - 1 : NV;
+    int k = CHECK ? KVX + grp : grp;
 #pragma unroll UNROLL
     for (; k < nr; k += NG) {
       double f[NS];
@@ -522,7 +556,10 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
     double* wl = plus + j * NT + t;
     double* wr = minus + (own ? (j + 1) * NT + t : t + W);
     double am;
-    face_one<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
+    if (CHECK)
+      face_check<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
+    else
+      face_one<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
     amax = am > amax ? am : amax;
   }
   return amax;
@@ -570,7 +607,7 @@ constexpr int sweep_minb(int lc) {
 // The sweeps of a stage in one launch: the blocks of the directions one after
 // another, so that the partial last wave of one overlaps the next.  They are
 // independent: each writes its own face fluxes and signal-speed slots.
-template <int KIND, int REC, int LC>
+template <int KIND, int REC, int LC, bool CHECK = false>
 __global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC)) sweep_kernel(const __grid_constant__ SweepArgs S) {
   extern __shared__ double sm[];
   constexpr int CPT = sweep_cpt<KIND>(LC), NG = (sweep_threads<KIND>(LC) * CPT) >> LC;
@@ -580,13 +617,13 @@ __global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC))
   int dir;
   if (b < S.first[1]) {
     dir = 0;
-    amax = face_tile<KIND, 0, REC, LC, CPT, NG>(S.A[0], b, S.lw, sm);
+    amax = face_tile<KIND, 0, REC, LC, CPT, NG, CHECK>(S.A[0], b, S.lw, sm);
   } else if (b < S.first[2]) {
     dir = 1;
-    amax = face_tile<KIND, 1, REC, LC, CPT, NG>(S.A[1], b - S.first[1], S.lw, sm);
+    amax = face_tile<KIND, 1, REC, LC, CPT, NG, CHECK>(S.A[1], b - S.first[1], S.lw, sm);
   } else {
     dir = 2;
-    amax = face_tile<KIND, 2, REC, LC, CPT, NG>(S.A[2], b - S.first[2], S.lw, sm);
+    amax = face_tile<KIND, 2, REC, LC, CPT, NG, CHECK>(S.A[2], b - S.first[2], S.lw, sm);
   }
   DevScalars* sc = S.A[0].sc;
   block_max_atomic(amax, &sc->amax_bits[dir], red);

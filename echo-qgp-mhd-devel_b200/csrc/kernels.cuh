@@ -1079,6 +1079,12 @@ __global__ void __launch_bounds__(128, ECHO_SSP_MINB) ssp_stage1_kernel(SspArgs 
     sp = seed;
   }
   if (!active) return;
+  {
+    // the EoS check of the right-hand side of U^n (system_source)
+    double en = 0.;
+    const int e = eos_energy(A.P, vv[KRH], &en, vv[KPR]);
+    if (e) atomicMin(&A.sc->err_key, ((unsigned long long)c << 20) | (unsigned long long)e);
+  }
   int it = 0, sfail = 0;
   int err = cons2prim<KIND>(A.P, M, A.algo, A.tol, uu, vv, &it, sp, &sfail, alpha_imex * A.sc->dt);
   if (SEED && (sfail & 1)) atomicAdd(&A.sc->fallbacks, 1ull);

@@ -2,6 +2,8 @@
 // included only by kind_*.cu, each of which instantiates one equation set.
 #pragma once
 
+#include <type_traits>
+
 #include "batch.cuh"
 #include "stage.cuh"
 
@@ -22,9 +24,10 @@ inline int sweep_lc(const EchoCtx* c, int mask) {
 }
 
 // the sweeps of the directions in mask (bit d: direction d), one launch; last,
-// if given: the stage's scalar logic by the block that finishes last
+// if given: the stage's scalar logic by the block that finishes last; check:
+// the faces' errors and signal speeds only (resistive runs)
 template <int KIND>
-void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last) {
+void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last, bool check) {
   SweepArgs S;
   memset(&S, 0, sizeof(S));
   if (last) {
@@ -58,13 +61,26 @@ void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last) {
     fn<<<blocks, sweep_threads<KIND>(lc), smem, c->stream>>>(S);
   };
   // the schemes in use get a kernel of their own; the others choose at run time
-  auto pick = [&](auto big, auto small) { lc == 8 ? go(big) : go(small); };
-  if (c->p.recal == ECHO_REC_WENO5)
-    pick(sweep_kernel<KIND, ECHO_REC_WENO5, 8>, sweep_kernel<KIND, ECHO_REC_WENO5, 5>);
-  else if (c->p.recal == ECHO_REC_MPE5)
-    pick(sweep_kernel<KIND, ECHO_REC_MPE5, 8>, sweep_kernel<KIND, ECHO_REC_MPE5, 5>);
-  else
-    pick(sweep_kernel<KIND, REC_RUNTIME, 8>, sweep_kernel<KIND, REC_RUNTIME, 5>);
+  auto pick = [&](auto rec, auto chk) {
+    constexpr int R = decltype(rec)::value;
+    constexpr bool K = decltype(chk)::value;
+    lc == 8 ? go(sweep_kernel<KIND, R, 8, K>) : go(sweep_kernel<KIND, R, 5, K>);
+  };
+  auto scheme = [&](auto chk) {
+    if (c->p.recal == ECHO_REC_WENO5)
+      pick(std::integral_constant<int, ECHO_REC_WENO5>(), chk);
+    else if (c->p.recal == ECHO_REC_MPE5)
+      pick(std::integral_constant<int, ECHO_REC_MPE5>(), chk);
+    else
+      pick(std::integral_constant<int, REC_RUNTIME>(), chk);
+  };
+  if constexpr (Traits<KIND>::RES) {
+    if (check) {
+      scheme(std::true_type());
+      return;
+    }
+  }
+  scheme(std::false_type());
 }
 
 template <int KIND>
@@ -674,7 +690,7 @@ void batch_occupancy(const EchoBatch* b, int* per_sm) {
 }  // namespace echo
 
 #define ECHO_INSTANTIATE_GRID(K)                                              \
-  template void echo::launch_faces<K>(EchoCtx*, int, const ScalarArgs*);                         \
+  template void echo::launch_faces<K>(EchoCtx*, int, const ScalarArgs*, bool);                         \
   template int echo::setup_stage<K>(EchoCtx*, int, int, int);                 \
   template void echo::launch_stage<K>(EchoCtx*, int, int, double*);           \
   template void echo::launch_update<K>(EchoCtx*, int, int, double*);          \
