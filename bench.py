@@ -733,7 +733,9 @@ def run_b200(args):
         flop_step = sum(krec[k]["fp64_flop"] * n for k, (_, n) in prof.items() if k in krec and n)
     counters_src = {"file": os.path.relpath(COUNTERS, ROOT), "build_hash": cnt.get("build_hash"),
                     "this_build": CT.build_hash(), "same_build": fresh}
-    launches_per_step = sum(n for (_, n) in prof.values())
+    # one launch each per stage: the sweeps (with the stage's scalars), the update,
+    # the repair (which also ends the step)
+    launches_per_step = 3 * cfg0.nrk
 
     cpu = None
     if world == 1:

@@ -1382,7 +1382,9 @@ __device__ int cons2prim(const DevPhys& P, const Metric& M, int algo, double tol
 }
 
 // ---------------------------------------------------------------------------
-// get_sigma (viscous.f90:283-393)
+// get_sigma (viscous.f90:283-393); the product build's Milne runs take it in
+// covariant form (visc_source_milne: 201 x 201 viscous update 49 -> 21 us with
+// the inversion's fluid_step)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void get_sigma(const DevPhys& P, const Metric& M, const double* v, const double* d,
                                           double sigma[6]) {

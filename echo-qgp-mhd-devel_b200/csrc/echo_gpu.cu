@@ -276,7 +276,7 @@ static void enqueue_stage_ssp(EchoCtx* c, int irk, int then) {
     // Resistive runs: only S(U1) of the first stage enters the combinations
     // (F(U1) has weight 0), so its sweeps check the faces and set the cleaning
     // speed, and its right-hand side is not formed (ssp_stage1_kernel keeps
-    // that one's EoS check).  193 x 193 x 129: 11.2 -> 9.6 ms a step.
+    // that one's EoS check).  193 x 193 x 129: 11.1 -> 9.8 ms a step.
     const bool check = irk == 1 && c->kind == KIND_RES;
     const ScalarArgs S = scalar_args(c, irk, 2, reset);
     launch_sweeps(c, &S, check);

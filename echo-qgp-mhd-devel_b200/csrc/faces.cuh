@@ -23,7 +23,7 @@
 //
 // Measured, x / y / eta us a launch, one thread per face before and this: ideal
 // RMHD 97 x 97 x 81 111 / 108 / 114 and 76 / 70 / 73; resistive 193 x 193 x 129
-// 742 / 733 / 844 and 451 / 498 / 520.  With the loads, the reconstruction or
+// 742 / 733 / 844 and 451 / 500 / 530.  With the loads, the reconstruction or
 // the flux left out in turn the RMHD x sweep took 62, 69 and 72 us: no one of
 // them bounds it.
 #pragma once

@@ -1,10 +1,11 @@
 // kernels.cuh -- the device kernels of one RK stage.
 //
-//   faces<KIND,DIR>   one thread per cell face along DIR: boundary ghosts,
+//   sweep_kernel<KIND> (faces.cuh) the flux sweeps: boundary ghosts,
 //                     reconstruction, the p<=0 / v^2>=1 fix-ups, GLM, two
 //                     system_flux calls and the HLL flux (evolve_df[xyz],
 //                     evolve.f90:302-685; work_fup[xyz], work.f90:143-416);
-//                     writes the face flux and the max signal speed.
+//                     writes the face flux and the max signal speed.  The
+//                     batched sweeps compute a face per thread (face_flux).
 //   stage_scalars     the scalar logic of evolve_main (dt, CFL reduction
 //                     result, GLM speed and damping factor).
 //   update<KIND>      one thread per cell: flux divergence + sources + RK

@@ -39,10 +39,11 @@ def build_hash() -> str:
     return h.hexdigest()[:16]
 
 
-def kernel_class(name: str) -> str | None:
-    if name.startswith("void faces_kernel<"):
-        d = name.split("<")[1].split(",")[1].strip()
-        return "faces_" + "xyz"[int(d)]
+def kernel_class(name: str, sweep: int) -> str | None:
+    """sweep: how many sweeps the capture holds before this launch (a capture
+    of ordered sweeps, `drive --ordered`, starting with an x sweep)."""
+    if name.startswith("void sweep_kernel<"):
+        return "faces_" + "xyz"[sweep % 3]
     if name.startswith("void update_kernel<"):
         return "update_c2p"
     if name.startswith("void stage_kernel<"):
@@ -63,9 +64,11 @@ def parse(report: str) -> dict:
     scale = {"byte": 1.0, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "nsecond": 1e-3, "usecond": 1.0,
              "msecond": 1e3, "second": 1e6}
     recs: dict[str, list[dict]] = {}
+    sweeps = 0
     for r in rows[2:]:
         d = dict(zip(hdr, r))
-        cls = kernel_class(d.get("Kernel Name", ""))
+        cls = kernel_class(d.get("Kernel Name", ""), sweeps)
+        sweeps += cls is not None and cls.startswith("faces_")
         if cls is None:
             continue
 

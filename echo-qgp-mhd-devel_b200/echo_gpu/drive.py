@@ -62,6 +62,7 @@ def main():
     ap.add_argument("--faces", type=int, default=-1, choices=[-1, 0, 8, 16],
                     help="product build face sweeps: 8/16 cells along a y or eta tile, 0 the library's choice "
                          "(-1: leave it)")
+    ap.add_argument("--ordered", action="store_true", help="the sweeps of a stage one launch after another")
     a = ap.parse_args()
     if a.config == "batch":
         run_batch(a)
@@ -92,6 +93,8 @@ def main():
         print(f"stage: {info}")
     if a.faces >= 0:
         ev.set_faces(a.faces)
+    if a.ordered:
+        ev.set_sweeps(False)
     ev.upload(I.primitives(cfg, tab), None, cfg.tstart)
     t0 = time.perf_counter()
     ev.run(a.steps)
