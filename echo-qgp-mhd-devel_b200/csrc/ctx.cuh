@@ -61,6 +61,7 @@ struct EchoCtx {
   int face_mode;
   // one launch for all the sweeps of a stage (1), or one each in order
   int par_sweeps;
+  int wide;  // sweeps with 64-bit byte offsets (wide_grid)
   // echo_gpu_advance_host: the host copy of u runs on copy_stream and ev_u
   // marks its end; while wait_u is set, the next step's first u access
   // waits for it (join_u)

@@ -439,6 +439,7 @@ int echo_gpu_init(const EchoParams* p, const double* eos_table, int n_eos, EchoC
   CK(cudaEventCreateWithFlags(&c->ev_u, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&c->ev_u_fork, cudaEventDisableTiming));
   c->par_sweeps = ECHO_PAR_SWEEPS;
+  c->wide = wide_grid(c->g);
   for (int i = 0; i < 2; i++) {
     CK(cudaMalloc(&c->d_v[i], sizeof(double) * nvc));
     CK(cudaMalloc(&c->d_u[i], sizeof(double) * nvc));
@@ -1006,6 +1007,19 @@ int echo_gpu_set_sweeps(EchoCtx* c, int concurrent) {
   if (!c || (concurrent != 0 && concurrent != 1)) return ECHO_ERR_ARG;
   CK(cudaStreamSynchronize(c->stream));
   c->par_sweeps = concurrent;
+  for (int i = 0; i < 16; i++)
+    if (c->graph_ok[i]) {
+      cudaGraphExecDestroy(c->graph[i]);
+      c->graph_ok[i] = false;
+    }
+  return ECHO_OK;
+}
+
+int echo_gpu_test_wide(EchoCtx* c) {
+  if (!c) return ECHO_ERR_ARG;
+  if (c->kind != KIND_HD) return ECHO_ERR_UNSUPPORTED;
+  CK(cudaStreamSynchronize(c->stream));
+  c->wide = 1;
   for (int i = 0; i < 16; i++)
     if (c->graph_ok[i]) {
       cudaGraphExecDestroy(c->graph[i]);

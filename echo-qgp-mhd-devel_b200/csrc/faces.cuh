@@ -54,8 +54,9 @@ __host__ __device__ constexpr size_t tile_smem(int lc) {
   return sizeof(double) * 2 * (size_t)tile_rows_of_states<KIND>() * ((size_t)1 << lc);
 }
 
-// tiles of a sweep of grid g (face and cell counts are below 2^32: the arrays
-// of a larger grid would not fit the device)
+// tiles of a sweep of grid g (cells, faces and the padded cells of x pencils, at
+// most twice the cells, are counted below 2^32: the arrays of the smallest run,
+// 1-D hydro, have 265 bytes a cell)
 __host__ __device__ inline unsigned tiles_of(const Grid& g, int dir, int lc, int lw) {
   const unsigned C = 1u << lc;
   if (dir == 0) {
@@ -65,6 +66,26 @@ __host__ __device__ inline unsigned tiles_of(const Grid& g, int dir, int lc, int
   const unsigned n = (unsigned)(dir == 1 ? g.ny : g.nz), cols = (unsigned)g.nx * (unsigned)(dir == 1 ? g.nz : g.ny);
   const unsigned rows = (C >> lw) - 1;
   return ((cols + (1u << lw) - 1) >> lw) * ((n + 1 + rows - 1) / rows);
+}
+
+// index of the face above cell c (0..n) of a pencil: its transverse position
+// (ta, tb), first cell base and stride
+template <int DIR>
+__host__ __device__ __forceinline__ unsigned face_index(const Grid& g, unsigned c, unsigned ta, unsigned tb,
+                                                        unsigned base, unsigned stride) {
+  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny;
+  return DIR == 0 ? (tb * ny + ta) * (nx + 1) + c : DIR == 1 ? (tb * (ny + 1) + c) * nx + ta : c * stride + base;
+}
+
+// Whether the sweeps of grid g need 64-bit byte offsets.  2^29 cells and more
+// fit the device in ideal hydro alone (265, 305 and 345 bytes a cell in 1-D, 2-D
+// and 3-D; the next set, 1-D RMHD, has 385).  Not always: the stencil's offsets
+// as 64-bit pairs cost the sweeps 0.5 to 1 % (75 x 67 x 49 hydro MPE5 1010 us
+// for 5 steps with 32 bits, 1021 with 64).
+inline bool wide_grid(const Grid& g) {
+  const size_t lim = (size_t)1 << 29;
+  return g.ncell > lim || (g.nx > 1 && faces_of<0>(g) > lim) || (g.ny > 1 && faces_of<1>(g) > lim) ||
+         (g.nz > 1 && faces_of<2>(g) > lim);
 }
 
 #ifndef ECHO_EXACT
@@ -301,7 +322,7 @@ static __device__ __noinline__ void fix_states(const FaceArgs& A, const Metric& 
 // The flux of the face above cell c of a pencil (base, stride) from its states
 // wl, wr (variable k at k * C; changed in place by the fix-ups and the GLM
 // upwinding): writes A.F (and A.WD), the signal speed into amax.
-template <int KIND, int DIR, int C>
+template <int KIND, int DIR, int C, bool WIDE>
 __device__ __forceinline__ void face_one(const FaceArgs& A, const Metric& M, unsigned base, unsigned stride, int n,
                                          int c, int ta, int tb, double* wl, double* wr, double& amax) {
   typedef Traits<KIND> T;
@@ -309,9 +330,7 @@ __device__ __forceinline__ void face_one(const FaceArgs& A, const Metric& M, uns
   const Grid& g = A.g;
   amax = 0.;
   const size_t nfaces = faces_of<DIR>(g);
-  const unsigned fid = DIR == 0   ? ((unsigned)tb * (unsigned)g.ny + (unsigned)ta) * (unsigned)(g.nx + 1) + (unsigned)c
-                       : DIR == 1 ? ((unsigned)tb * (unsigned)(g.ny + 1) + (unsigned)c) * (unsigned)g.nx + (unsigned)ta
-                                  : (unsigned)c * stride + base;
+  const unsigned fid = face_index<DIR>(g, (unsigned)c, (unsigned)ta, (unsigned)tb, base, stride);
   if (T::VISC) {
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -374,7 +393,7 @@ __device__ __forceinline__ void face_one(const FaceArgs& A, const Metric& M, uns
     for (int k = 0; k < NV; k++) F[k] = 0.0;
   }
 #pragma unroll
-  for (int k = 0; k < NV; k++) *(double*)((char*)(A.F + (size_t)k * nfaces) + 8u * fid) = F[k];
+  for (int k = 0; k < NV; k++) *(double*)((char*)(A.F + (size_t)k * nfaces) + off8<WIDE>(fid)) = F[k];
   if (!err) {
     // GLM speed of the reference: the last face of the last pencil (work.f90:217,310,401)
     const int na = DIR == 0 ? g.ny : g.nx, nb = DIR == 2 ? g.ny : g.nz;
@@ -419,8 +438,9 @@ __device__ __forceinline__ void face_check(const FaceArgs& A, const Metric& M, u
 // One tile of the sweep along DIR; returns the largest signal speed of this
 // thread's faces.  Called by every thread of the block: NG groups of C / CPT
 // threads, the groups sharing the variables of phase 1.  sm:
-// tile_smem<KIND>(LC) bytes.  CHECK: velocity and pressure, face_check.
-template <int KIND, int DIR, int REC, int LC, int CPT, int NG, bool CHECK>
+// tile_smem<KIND>(LC) bytes.  CHECK: velocity and pressure, face_check.  WIDE:
+// wide_grid.
+template <int KIND, int DIR, int REC, int LC, int CPT, int NG, bool CHECK, bool WIDE>
 __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, int lw, double* sm) {
   typedef Traits<KIND> T;
   constexpr int NV = T::NV, C = 1 << LC, NT = C / CPT, NS = CPT + 4, UNROLL = ECHO_SWEEP_UNROLL;
@@ -436,9 +456,7 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
   const double mt = A.sc->t, mt3 = A.sc->t3;
 
   // this thread's first cell: pencil index c (0 and n + 1 are the ghosts next
-  // to the grid), first cell and stride of its pencil, transverse position.
-  // Cell and face indices are below 2^29 (their doubles' byte offsets below
-  // 2^32): the arrays of a larger grid do not fit the device.
+  // to the grid), first cell and stride of its pencil, transverse position
   int c, ta, tb;
   unsigned base;
   bool ok;
@@ -468,18 +486,18 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
     // byte offsets of the stencil from cell c - 2 on, with the ghost fill of
     // evolve_bc[xyz]; the last cell's own upper neighbour is not read
     const int last = c + CPT - 1 <= n + 1 ? NS - 1 : NS - 2;
-    unsigned off[NS];
+    Off<WIDE> off[NS];
     int neg = 0;
     if (c >= 3 && c + CPT + 1 <= n) {
 #pragma unroll
-      for (int q = 0; q < NS; q++) off[q] = 8u * (base + (unsigned)(c - 3 + q) * stride);
+      for (int q = 0; q < NS; q++) off[q] = off8<WIDE>(base + (unsigned)(c - 3 + q) * stride);
     } else {
 #pragma unroll
       for (int q = 0; q < NS; q++) {
         int qq;
         double sg;
         map_ghost(c - 2 + (q < last ? q : last), n, A.bc.c[0][0], A.bc.c[0][1], qq, sg);
-        off[q] = 8u * (base + (unsigned)(qq - 1) * stride);
+        off[q] = off8<WIDE>(base + (unsigned)(qq - 1) * stride);
         if (sg < 0.) neg |= 1 << q;
       }
     }
@@ -559,7 +577,7 @@ __device__ __forceinline__ double face_tile(const FaceArgs& A, unsigned tile, in
     if (CHECK)
       face_check<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
     else
-      face_one<KIND, DIR, C>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
+      face_one<KIND, DIR, C, WIDE>(A, M, base, stride, n, cf, ta, tb, wl, wr, am);
     amax = am > amax ? am : amax;
   }
   return amax;
@@ -607,7 +625,7 @@ constexpr int sweep_minb(int lc) {
 // The sweeps of a stage in one launch: the blocks of the directions one after
 // another, so that the partial last wave of one overlaps the next.  They are
 // independent: each writes its own face fluxes and signal-speed slots.
-template <int KIND, int REC, int LC, bool CHECK = false>
+template <int KIND, int REC, int LC, bool CHECK = false, bool WIDE = false>
 __global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC)) sweep_kernel(const __grid_constant__ SweepArgs S) {
   extern __shared__ double sm[];
   constexpr int CPT = sweep_cpt<KIND>(LC), NG = (sweep_threads<KIND>(LC) * CPT) >> LC;
@@ -617,13 +635,13 @@ __global__ void __launch_bounds__(sweep_threads<KIND>(LC), sweep_minb<KIND>(LC))
   int dir;
   if (b < S.first[1]) {
     dir = 0;
-    amax = face_tile<KIND, 0, REC, LC, CPT, NG, CHECK>(S.A[0], b, S.lw, sm);
+    amax = face_tile<KIND, 0, REC, LC, CPT, NG, CHECK, WIDE>(S.A[0], b, S.lw, sm);
   } else if (b < S.first[2]) {
     dir = 1;
-    amax = face_tile<KIND, 1, REC, LC, CPT, NG, CHECK>(S.A[1], b - S.first[1], S.lw, sm);
+    amax = face_tile<KIND, 1, REC, LC, CPT, NG, CHECK, WIDE>(S.A[1], b - S.first[1], S.lw, sm);
   } else {
     dir = 2;
-    amax = face_tile<KIND, 2, REC, LC, CPT, NG, CHECK>(S.A[2], b - S.first[2], S.lw, sm);
+    amax = face_tile<KIND, 2, REC, LC, CPT, NG, CHECK, WIDE>(S.A[2], b - S.first[2], S.lw, sm);
   }
   DevScalars* sc = S.A[0].sc;
   block_max_atomic(amax, &sc->amax_bits[dir], red);

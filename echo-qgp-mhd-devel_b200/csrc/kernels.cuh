@@ -17,6 +17,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "c2p.cuh"
 
 namespace echo {
@@ -73,6 +75,16 @@ __host__ __device__ inline void set_grid_div(Grid& g) {
   g.dnx1 = make_fastdiv((unsigned)g.nx + 1u);
   g.dny1 = make_fastdiv((unsigned)g.ny + 1u);
   g.dnx2 = make_fastdiv(((unsigned)g.nx + 3u) & ~1u);
+}
+
+// Byte offset of element i (counted below 2^32, FastDiv) of an array of doubles.
+// With 32 bits a load takes it as it is beside a 64-bit base, for arrays of at
+// most 2^29 elements; 64 bits (WIDE) hold every offset.
+template <bool WIDE>
+using Off = std::conditional_t<WIDE, size_t, unsigned>;
+template <bool WIDE>
+__host__ __device__ __forceinline__ Off<WIDE> off8(unsigned i) {
+  return (Off<WIDE>)i * 8u;
 }
 
 // boundary codes for one sweep direction: bc[k][side]
@@ -711,10 +723,11 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
   unsigned my_iters = 0, my_fallbacks = 0, my_brackets = 0;
   const Metric M = make_metric(A.coordinates, A.sc->t, A.sc->t3);
   double vv[NV], uu[NV];
+  const size_t c8 = off8<true>((unsigned)c);
   if (active) {
     double src[NV], kap[2] = {0., 0.};
 #pragma unroll
-    for (int k = 0; k < NV; k++) vv[k] = *(const double*)((const char*)(A.vin + (size_t)k * g.ncell) + 8u * (unsigned)c);
+    for (int k = 0; k < NV; k++) vv[k] = *(const double*)((const char*)(A.vin + (size_t)k * g.ncell) + c8);
     if (T::VISC) {
       if (A.vsnap) {
 #pragma unroll
@@ -786,7 +799,6 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
                                     T::RES ? stiff : nullptr);
       if (err) atomicMin(&A.sc->err_key, ((unsigned long long)c << 20) | (unsigned long long)err);
     }
-    const unsigned c8 = 8u * (unsigned)c;  // cell indices are below 2^29 (face_tile)
     auto at = [&](auto* a, int k) { return (decltype(a))((char*)(a + (size_t)k * g.ncell) + c8); };
     if (A.mode == MODE_RHS) {
 #pragma unroll
@@ -854,7 +866,7 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
         atomicAdd(&A.sc->nfail, 1);
       } else {
 #pragma unroll
-        for (int k = 0; k < NV; k++) *(double*)((char*)(A.vout + (size_t)k * g.ncell) + 8u * (unsigned)c) = vv[k];
+        for (int k = 0; k < NV; k++) *(double*)((char*)(A.vout + (size_t)k * g.ncell) + c8) = vv[k];
       }
     }
     // per-warp sums of iteration counts, seed and bracketed fallbacks
@@ -878,40 +890,43 @@ __device__ __forceinline__ void update_cell(const UpdateArgs& A, size_t c, bool 
   int ix = 0, iy = 0, iz = 0;
   double du[NV], dv[NDER];
   // byte offsets of the cell's lower x, y and eta faces (faces ix, iy, iz of
-  // its pencils); face indices are below 2^29 (face_tile)
-  unsigned fx = 0, fy = 0, fz = 0;
-  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, sy = 8u * nx, sz = 8u * nx * ny;
+  // its pencils), 64-bit: a 2-D hydro run holds 305 bytes a cell, so that 2^29
+  // cells and more fit the device (97 x 97 x 81 RMHD update 304 us a step with
+  // 32 and with 64 bits)
+  size_t fx = 0, fy = 0, fz = 0;
+  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny;
+  const size_t sy = off8<true>(nx), sz = off8<true>(nx * ny);
   const size_t nfx = faces_of<0>(g), nfy = faces_of<1>(g), nfz = faces_of<2>(g);
-  auto up = [](const double* a, size_t k, unsigned off) { return *(const double*)((const char*)(a + k) + off); };
+  auto up = [](const double* a, size_t k, size_t off) { return *(const double*)((const char*)(a + k) + off); };
   if (active) {
     const unsigned cc = (unsigned)c, r = fast_div(cc, g.dnx), q = fast_div(r, g.dny);
     ix = (int)(cc - r * nx);
     iy = (int)(r - q * ny);
     iz = (int)q;
-    fx = 8u * (r * (nx + 1) + (unsigned)ix);
-    fy = 8u * ((q * (ny + 1) + (unsigned)iy) * nx + (unsigned)ix);
-    fz = 8u * cc;
+    fx = off8<true>(r * (nx + 1) + (unsigned)ix);
+    fy = off8<true>((q * (ny + 1) + (unsigned)iy) * nx + (unsigned)ix);
+    fz = off8<true>(cc);
     // flux divergence in the reference's order, du = 0; += x; += y; += z; the
     // loads of a direction together, one trip to memory each
 #pragma unroll
     for (int k = 0; k < NV; k++) du[k] = 0.;
-    auto flux = [&](const double* F, size_t nf, unsigned f, unsigned s, double dd) {
+    auto flux = [&](const double* F, size_t nf, size_t f, size_t s, double dd) {
 #pragma unroll
       for (int k = 0; k < NV; k++) du[k] = du[k] + dd * (up(F, k * nf, f + s) - up(F, k * nf, f));
     };
-    if (g.nx > 1) flux(A.Fx, nfx, fx, 8u, g.ddx);
+    if (g.nx > 1) flux(A.Fx, nfx, fx, 8, g.ddx);
     if (g.ny > 1) flux(A.Fy, nfy, fy, sy, g.ddy);
     if (g.nz > 1) flux(A.Fz, nfz, fz, sz, g.ddz);
     if (T::VISC) {
 #pragma unroll
       for (int i = 0; i < NDER; i++) dv[i] = 0.;
       const int dk[3][4] = {{DTX, DXX, DYX, DZX}, {DTY, DXY, DYY, DZY}, {DTZ, DXZ, DYZ, DZZ}};
-      auto grad = [&](const double* W, size_t nf, unsigned f, unsigned s, int i) {
+      auto grad = [&](const double* W, size_t nf, size_t f, size_t s, int i) {
         return up(W, i * nf, f + s) + up(W, (4 + i) * nf, f + s) - up(W, i * nf, f) - up(W, (4 + i) * nf, f);
       };
       if (g.nx > 1) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) dv[dk[0][i]] = g.ddx * 0.5 * grad(A.WDx, nfx, fx, 8u, i);
+        for (int i = 0; i < 4; i++) dv[dk[0][i]] = g.ddx * 0.5 * grad(A.WDx, nfx, fx, 8, i);
       }
       if (g.ny > 1) {
 #pragma unroll
@@ -978,8 +993,8 @@ __global__ void __launch_bounds__(128, ECHO_SSP_MINB) ssp_combine_kernel(SspArgs
   const double dt = A.sc->dt;
   if (active) {
     // the branch on the stage outside the loops, so that a stage's loads go
-    // out together; byte offsets below 2^32 (face_tile)
-    const unsigned c8 = 8u * (unsigned)c;
+    // out together
+    const size_t c8 = off8<true>((unsigned)c);
     auto at = [&](const double* a, int k) { return *(const double*)((const char*)(a + (size_t)k * g.ncell) + c8); };
     // stiff right-hand sides: zero but for E of resistive runs
     auto stiff = [&](const double* a, int k) { return T::RES && k >= KEX && k <= KEZ ? at(a, k - KEX) : 0.0; };

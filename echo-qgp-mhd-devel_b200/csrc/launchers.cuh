@@ -17,6 +17,7 @@ namespace echo {
 // where it does not (201 x 201 viscous x / y sweep 28 / 25 us with 32 cells,
 // 25 / 23 with 256; 101 x 101 hydro 12 / 9 and 14 / 12).
 inline int sweep_lc(const EchoCtx* c, int mask) {
+  if (c->wide) return 8;
   unsigned t = 0;
   for (int d = 0; d < 3; d++)
     if (mask >> d & 1) t += tiles_of(c->g, d, 8, 4);
@@ -64,6 +65,12 @@ void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last, bool check) {
   auto pick = [&](auto rec, auto chk) {
     constexpr int R = decltype(rec)::value;
     constexpr bool K = decltype(chk)::value;
+    if constexpr (KIND == KIND_HD) {
+      if (c->wide) {
+        go(sweep_kernel<KIND, R, 8, K, true>);
+        return;
+      }
+    }
     lc == 8 ? go(sweep_kernel<KIND, R, 8, K>) : go(sweep_kernel<KIND, R, 5, K>);
   };
   auto scheme = [&](auto chk) {

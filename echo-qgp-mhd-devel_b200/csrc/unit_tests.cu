@@ -93,6 +93,24 @@ extern "C" int echo_gpu_test_fastdiv(const unsigned* d, int nd, const unsigned* 
   return ECHO_OK;
 }
 
+extern "C" int echo_gpu_test_offsets(int nx, int ny, int nz, unsigned long long* off) {
+  if (nx < 1 || ny < 1 || nz < 1 || !off) return ECHO_ERR_ARG;
+  echo::Grid g;
+  memset(&g, 0, sizeof(g));
+  g.nx = nx;
+  g.ny = ny;
+  g.nz = nz;
+  g.ncell = (size_t)nx * ny * nz;
+  const unsigned x = (unsigned)nx, y = (unsigned)ny, z = (unsigned)nz;
+  const unsigned i[4] = {(unsigned)(g.ncell - 1), echo::face_index<0>(g, x, y - 1, z - 1, (z * y - 1) * x, 1),
+                         echo::face_index<1>(g, y, x - 1, z - 1, (z - 1) * x * y + x - 1, x),
+                         echo::face_index<2>(g, z, x - 1, y - 1, x * y - 1, x * y)};
+  const bool wide = echo::wide_grid(g);
+  for (int q = 0; q < 4; q++) off[q] = wide ? echo::off8<true>(i[q]) : echo::off8<false>(i[q]);
+  off[4] = echo::off8<true>(i[0]);  // the updates' (always 64-bit)
+  return ECHO_OK;
+}
+
 extern "C" int echo_gpu_test_recon(int recal, int m, int n, const double* f, double* gl, double* gr) {
   (void)cudaGetLastError();  // a failed launch of an earlier call must not be reported here
   if (m <= 0 || n <= 0 || !f || !gl || !gr) return ECHO_ERR_ARG;

@@ -108,6 +108,9 @@ FUNCTIONS = {
     "echo_gpu_advance_host": (ctypes.c_int, [P, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                              ctypes.c_void_p, ctypes.c_int]),
     "echo_gpu_test_recon": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, D, D, D]),
+    "echo_gpu_test_offsets": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                             ctypes.POINTER(ctypes.c_ulonglong)]),
+    "echo_gpu_test_wide": (ctypes.c_int, [P]),
     "echo_gpu_test_fastdiv": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
                                              ctypes.c_void_p]),
     "echo_gpu_test_c2p": (ctypes.c_int, [P, D, ctypes.c_int, ctypes.c_int, ctypes.c_double,
@@ -434,6 +437,16 @@ def unit_fastdiv(d, n, exact: bool = False):
     if rc:
         raise RuntimeError(f"test_fastdiv status {rc}")
     return q
+
+
+def unit_offsets(nx: int, ny: int, nz: int, exact: bool = False) -> list[int]:
+    """Byte offsets of the last cell, x, y and eta face in the sweeps of an
+    nx x ny x nz grid and of the last cell in its updates (host arithmetic)."""
+    off = (ctypes.c_ulonglong * 5)()
+    rc = load(exact).echo_gpu_test_offsets(nx, ny, nz, off)
+    if rc:
+        raise RuntimeError(f"test_offsets status {rc}")
+    return list(off)
 
 
 def unit_c2p(params, eos_table, g3, gp, u, vguess, exact: bool = True):

@@ -397,6 +397,15 @@ int echo_gpu_fp64_peak(double* gflops, double* ms);
  * to split flat indices into grid coordinates. */
 int echo_gpu_test_fastdiv(const unsigned* d, int nd, const unsigned* n, int nn, unsigned* q);
 
+/* Byte offsets (host) as the kernels form them on an nx x ny x nz grid: off[0]
+ * to off[3] the last cell, x face, y face and eta face of a variable in the
+ * sweeps, off[4] the last cell in the updates. */
+int echo_gpu_test_offsets(int nx, int ny, int nz, unsigned long long* off);
+
+/* An ideal-hydro context runs the sweeps with the 64-bit offsets that grids of
+ * more than 2^29 cells or faces take, whatever its grid. */
+int echo_gpu_test_wide(EchoCtx* ctx);
+
 /* Reconstruction of m pencils of length n (+ghosts) with REC_ALGO.
  * f is m rows of (n + 8) values, f[row*(n+8) + (i+4)] = f(i), i=-4..n+3;
  * gl/gr are m rows of n+1 faces (holib.f90:47-348). */
