@@ -739,7 +739,7 @@ static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, doubl
     double en = 0, dedp = 0;
     const double rh = P.eqstate == ECHO_EOS_IDEALGAS ? s.D * sqrt(1. - xx) : 0.;  // e depends on rho there only
     if (eos_energy_slope_at(P, rh, pp, &en, &dedp, at)) return -1;
-    const double ib = yy + s.B2, ib2 = ib * ib, iy = rcp_h3(yy), i1x = rcp_h3(1. - xx);
+    const double ib = yy + s.B2, ib2 = ib * ib, iy = rcp_n(yy), i1x = rcp_n(1. - xx);
     const double q2 = s.SB2 * (iy * iy), q3 = q2 * iy;
     const double F1 = ib2 * xx - q2 * (2 * yy + s.B2) - s.S2;
     const double F2 = yy - pp + 0.5 * (1. + xx) * s.B2 - 0.5 * q2 - s.U;
@@ -750,7 +750,7 @@ static __device__ int newton3(const DevPhys& P, const Sist3& s, double* X, doubl
     const double A = J31 + J33 * J21, B = 1. + J33 * J22, R = -(F3 + J33 * F2);
     const double det = ib2 * B - J12 * A;
     if (det == 0.0 || !isfinite(det)) return -1;
-    const double idet = rcp_h3(det);
+    const double idet = rcp_n(det);
     const double dx = -(F1 * B + J12 * R) * idet, dy = (ib2 * R + F1 * A) * idet;
     const double dp = F2 + J21 * dx + J22 * dy;
     if (done) {  // converged: polish and stop
@@ -856,11 +856,14 @@ __device__ __forceinline__ bool fluid_step(const DevPhys& P, double d, double s2
   // two reciprocals a step (w, the derivative) and no square root: rho enters
   // p only through dp/drho, which is zero but for the ideal gas; the callers
   // take it after the last step (fluid_rho)
-  const double rw = rcp_h3(w);
+  const double rw = rcp_n(w);
   v2 = s2 * (rw * rw);
-  if (v2 >= 1. || w == 0.) {
-    v2 = 1.;
-    return true;
+  if (!(v2 < 1.)) {
+    if (is_nan(v2)) {  // w is 0 or infinite: the division's infinity or 0
+      const double x = rcp_approx(w);
+      v2 = s2 * (x * x);
+    }
+    if (v2 >= 1.) return true;
   }
   const double i1 = 1. - v2, en = w * i1 - pr - extra;
   double df;
@@ -872,7 +875,7 @@ __device__ __forceinline__ bool fluid_step(const DevPhys& P, double d, double s2
     errcode = eos_pressure_it(P, 0., en, &n.pe, &n.dprdrh, &n.dprden, n.at);
     df = fma(n.dprden, v2, -1.);
   }
-  dpr = (pr - n.pe) * rcp_h3(df);
+  dpr = (pr - n.pe) * rcp_n(df);  // dp/de v^2 < 1
 #endif
   return false;
 }
@@ -1461,7 +1464,7 @@ __device__ __forceinline__ int visc_source_milne(const DevPhys& P, const Metric&
   if (at.h) {
     // get_viscous_parameters in the interval of e(p): T beside it in the table
     const double h = en + v[KPR], t1 = __ldg(P.tT + at.h - 2), t2 = __ldg(P.tT + at.h - 1);
-    const double temp = fma(t2 - t1, (v[KPR] - at.p0) * rcp_h3(at.hi - at.p0), t1);
+    const double temp = fma(t2 - t1, (v[KPR] - at.p0) * rcp_n(at.hi - at.p0), t1);
     if (en < P.emin) return 131;
     if (en > P.emax) return 132;
     eta = P.init_type == 2 ? P.eta_over_s : 0.197326 * P.eta_over_s * (h * rcp_h3(temp));

@@ -108,7 +108,7 @@ __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, co
   if (err) return err;
   const double v2 = vx * vx + vy * vy + M.g3 * (vz * vz);
   if (v2 > 1) return 333;
-  const double i1 = 1. - v2, glf = rsqrt_h3(i1), h = en + pr;
+  const double i1 = 1. - v2, glf = rsqrt_n(i1), h = en + pr;
   s.ww = (T::VISC ? h + w[KPIBU * ld] : h) * (glf * glf);
   s.D = rh * glf;
   s.em = 0.;
@@ -145,12 +145,12 @@ __device__ __forceinline__ int side_speeds(const DevPhys& P, const Metric& M, co
   // of equal terms, and the last bits of the speeds are its noise
   double a2 = cs2;
   if (T::MHD) {
-    const double ca2 = div_h3(b, b + h);
+    const double ca2 = div_n(b, b + h);
     a2 = cs2 + ca2 - cs2 * ca2;
   }
-  const double x = 1. - v2 * a2, den = div_h3(1., x), hd = DIR == 3 ? over_g3(M, x) : x;
+  const double x = 1. - v2 * a2, den = div_n(1., x), hd = DIR == 3 ? over_g3(M, x) : x;
   const double vf1 = den * (1. - a2) * vd;
-  const double vf2 = den * sqrt_h3(a2 * i1 * (hd - (1. - a2) * (vd * vd)));
+  const double vf2 = den * sqrt_n(a2 * i1 * (hd - (1. - a2) * (vd * vd)));
   vfp = vf1 + vf2;
   vfm = vf1 - vf2;
   return 0;
@@ -262,7 +262,7 @@ __device__ __forceinline__ void hll_flux(const DevPhys& P, const Metric& M, cons
                                          const FaceSide& L, const FaceSide& R, double ap, double am, double* F) {
   double a1 = 1.;
   if (!(ap == 0. && am == 0.)) {
-    a1 = div_h3(1., ap + am);
+    a1 = div_n(1., ap + am);
   }
 #pragma unroll
   for (int k = 0; k < Traits<KIND>::NV; k++) F[k] = 0.;

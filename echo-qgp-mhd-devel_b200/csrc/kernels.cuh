@@ -757,7 +757,7 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
 #else
         const double gamma1 = rsqrt_h3(1. - vxo * vxo - vyo * vyo - A.sc->g3old * (vzo * vzo));
         const double gamma2 = rsqrt_h3(1. - vx * vx - vy * vy - M.g3 * (vz * vz));
-        const double iti = rcp_h3(ti);
+        const double iti = rcp_n(ti);
         dv[DTT] = (gamma2 - gamma1) * iti;
         dv[DXT] = (gamma2 * vx - gamma1 * vxo) * iti;
         dv[DYT] = (gamma2 * vy - gamma1 * vyo) * iti;
@@ -835,7 +835,7 @@ __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, boo
 #ifdef ECHO_EXACT
           uu[k] = (A.c1 * u0[k] + A.c2 * (ui - dt * d) + ck * ui) / (1. + ck);
 #else
-          uu[k] = (A.c1 * u0[k] + A.c2 * (ui - dt * d) + ck * ui) * rcp_h3(1. + ck);
+          uu[k] = (A.c1 * u0[k] + A.c2 * (ui - dt * d) + ck * ui) * rcp_n(1. + ck);
 #endif
         } else {
           uu[k] = A.c1 * u0[k] + A.c2 * (ui - dt * d);

@@ -145,35 +145,66 @@ __device__ __forceinline__ double over_gp(const Metric& M, double x) {
 
 #ifndef ECHO_EXACT
 // ---------------------------------------------------------------------------
-// Reciprocal, reciprocal square root and square root of the product build:
-// the hardware's approximation (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64)
-// and one third-order Householder correction each (Householder, The Numerical
-// Treatment of a Single Nonlinear Equation, 1970, ch. 4: x (1 + e + e^2) for
-// 1/a with e = 1 - a x, y (1 + e/2 + 3 e^2 / 8) for 1/sqrt(a) with
-// e = 1 - a y^2), without the special-case branches of the division and of
-// sqrt().  For normal a whose reciprocal is normal too; the callers' operands
-// are (denominators of the WENO weights, 1 - v^2, wave-speed sums).
+// Reciprocal, reciprocal square root, square root and quotient of the product
+// build: the hardware's approximation (PTX rcp.approx.ftz.f64,
+// rsqrt.approx.ftz.f64, relative errors of about 2^-23) and one third-order
+// Householder correction each (Householder, The Numerical Treatment of a Single
+// Nonlinear Equation, 1970, ch. 4: x (1 + e + e^2) for 1/a with e = 1 - a x,
+// y (1 + e/2 + 3 e^2 / 8) for 1/sqrt(a) with e = 1 - a y^2), without the
+// special-case branches of the division and of sqrt().
+//
+// Errors over normal operands and results: reciprocal, square root and quotient
+// within 0.51 ulp, rsqrt within 1.01 (the rounding of a y enters e).
+//
+// *_h3 return the division's and sqrt's own results at 0, infinity and NaN: a
+// con2prim that starts at v^2 = 1 or from no pressure meets 1 - v^2 = 0 and an
+// infinite or zero enthalpy.  There the correction is NaN (of 0 times infinity)
+// and the approximation the result.  Subnormal operands and results count as 0;
+// the square roots take operands below 1e-290 as 0.
+//
+// *_n, where operands and results are normal or a NaN is as good as the
+// division's result: the WENO weights' denominators, the speeds of a face state
+// (v^2 < 1), table spacings, the Newton steps of newton3 (which leave NaN to
+// BRENTM).  With the test for NaN in the speeds and in newton3 too a step of
+// 97 x 97 x 81 RMHD took 965 us, 954 without it there.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double rcp_h3(double a) {
+__device__ __forceinline__ bool is_nan(double r) { return (unsigned)__double2hiint(r) << 1 > 0xffe00000u; }
+__device__ __forceinline__ double rcp_approx(double a) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+  return x;
+}
+__device__ __forceinline__ double rsqrt_approx(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+  return y;
+}
+__device__ __forceinline__ double rcp_step(double a, double x) {
   const double e = fma(-a, x, 1.);
   return fma(x, fma(e, e, e), x);
 }
-__device__ __forceinline__ double rsqrt_h3(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+__device__ __forceinline__ double rsqrt_step(double a, double y) {
   const double e = fma(-a * y, y, 1.);
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
-// sqrt(a); arguments below 1e-290 (zero: a state without sound) give 0
-__device__ __forceinline__ double sqrt_h3(double a) {
-  const double y = rsqrt_h3(a), r = a * y;
+__device__ __forceinline__ double rcp_n(double a) { return rcp_step(a, rcp_approx(a)); }
+__device__ __forceinline__ double rcp_h3(double a) {
+  const double x = rcp_approx(a), r = rcp_step(a, x);
+  return is_nan(r) ? x : r;
+}
+__device__ __forceinline__ double rsqrt_n(double a) { return rsqrt_step(a, rsqrt_approx(a)); }
+__device__ __forceinline__ double rsqrt_h3(double a) {
+  const double y = rsqrt_approx(a), r = rsqrt_step(a, y);
+  return is_nan(r) ? y : r;
+}
+__device__ __forceinline__ double sqrt_n(double a) {
+  const double y = rsqrt_n(a), r = a * y;
   return fabs(a) < 1e-290 ? 0. : fma(fma(-r, r, a), 0.5 * y, r);
 }
-// b / a, the quotient of rcp_h3 corrected by its residual
-__device__ __forceinline__ double div_h3(double b, double a) {
-  const double x = rcp_h3(a), q = b * x;
+__device__ __forceinline__ double sqrt_h3(double a) { return __double2hiint(a) == 0x7ff00000 ? a : sqrt_n(a); }
+// b / a, the quotient of rcp_n corrected by its residual
+__device__ __forceinline__ double div_n(double b, double a) {
+  const double x = rcp_n(a), q = b * x;
   return fma(fma(-q, a, b), x, q);
 }
 #endif
@@ -591,7 +622,7 @@ __device__ __forceinline__ void weno5_cell(double f1, double f2, double f3, doub
   double np, mp, nm, mm;
   weno5_nm(Da, Dc, g, H, wbc, wac, wab, np, mp);
   weno5_nm(Dc, Da, g, H, wab, wac, wbc, nm, mm);  // reversed: the first differences change sign
-  const double inv = 0.375 * rcp_h3(mp * mm);
+  const double inv = 0.375 * rcp_n(mp * mm);
   plus = f3 + fma(np * mm, inv, 0.5 * d1);  // one rounding at the size of f3
   minus = f3 + fma(nm * mp, inv, -0.5 * d2);
 }
@@ -620,7 +651,7 @@ __device__ __forceinline__ void weno5_pair(const double f[6], double plus[2], do
     double np, mp, nm, mm;
     weno5_nm(Da, Dc, g, H, wbc, wac, wab, np, mp);
     weno5_nm(Dc, Da, g, H, wab, wac, wbc, nm, mm);
-    const double inv = 0.375 * rcp_h3(mp * mm);
+    const double inv = 0.375 * rcp_n(mp * mm);
     plus[c] = f[c + 2] + fma(np * mm, inv, 0.5 * d[c + 1]);
     minus[c] = f[c + 2] + fma(nm * mp, inv, -0.5 * d[c + 2]);
   }
@@ -642,7 +673,7 @@ __device__ __forceinline__ void weno5_face(const double s[6], double& gl, double
   Q3 = q3 * q3;
   w = Q1 * Q3;
   weno5_nm(D4, D2, w * D3, (20. / 3.) * D3, Q2 * Q3, w, Q1 * Q2, nr, mr);
-  const double inv = 0.375 * rcp_h3(ml * mr);
+  const double inv = 0.375 * rcp_n(ml * mr);
   gl = s[2] + fma(nl * mr, inv, 0.5 * d1);
   gr = s[3] + fma(nr * ml, inv, -0.5 * d3);
 }

@@ -93,6 +93,42 @@ extern "C" int echo_gpu_test_fastdiv(const unsigned* d, int nd, const unsigned* 
   return ECHO_OK;
 }
 
+// product build: the reciprocals of physics.cuh; parity build: CUDA's operators
+static __global__ void recip_test_kernel(int op, int n, const double* a, const double* b, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+#ifdef ECHO_EXACT
+  out[i] = op == 1 || op == 5 ? 1. / sqrt(a[i]) : op == 2 || op == 6 ? sqrt(a[i]) : op == 3 ? b[i] / a[i] : 1. / a[i];
+#else
+  out[i] = op == 0   ? echo::rcp_h3(a[i])
+           : op == 1 ? echo::rsqrt_h3(a[i])
+           : op == 2 ? echo::sqrt_h3(a[i])
+           : op == 3 ? echo::div_n(b[i], a[i])
+           : op == 4 ? echo::rcp_n(a[i])
+           : op == 5 ? echo::rsqrt_n(a[i])
+                     : echo::sqrt_n(a[i]);
+#endif
+}
+
+extern "C" int echo_gpu_test_recip(int op, int n, const double* a, const double* b, double* out) {
+  (void)cudaGetLastError();
+  if (op < 0 || op > 6 || n <= 0 || !a || !b || !out) return ECHO_ERR_ARG;
+  const size_t nb = (size_t)n * sizeof(double);
+  double *da, *db, *dc;
+  CK(cudaMalloc(&da, nb));
+  CK(cudaMalloc(&db, nb));
+  CK(cudaMalloc(&dc, nb));
+  CK(cudaMemcpy(da, a, nb, cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(db, b, nb, cudaMemcpyHostToDevice));
+  recip_test_kernel<<<(n + 127) / 128, 128>>>(op, n, da, db, dc);
+  CK(cudaGetLastError());
+  CK(cudaMemcpy(out, dc, nb, cudaMemcpyDeviceToHost));
+  cudaFree(da);
+  cudaFree(db);
+  cudaFree(dc);
+  return ECHO_OK;
+}
+
 extern "C" int echo_gpu_test_offsets(int nx, int ny, int nz, unsigned long long* off) {
   if (nx < 1 || ny < 1 || nz < 1 || !off) return ECHO_ERR_ARG;
   echo::Grid g;

@@ -110,6 +110,7 @@ FUNCTIONS = {
     "echo_gpu_test_recon": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, D, D, D]),
     "echo_gpu_test_offsets": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                              ctypes.POINTER(ctypes.c_ulonglong)]),
+    "echo_gpu_test_recip": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, D, D, D]),
     "echo_gpu_test_wide": (ctypes.c_int, [P]),
     "echo_gpu_test_fastdiv": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
                                              ctypes.c_void_p]),
@@ -437,6 +438,19 @@ def unit_fastdiv(d, n, exact: bool = False):
     if rc:
         raise RuntimeError(f"test_fastdiv status {rc}")
     return q
+
+
+def unit_recip(op: int, a, b=None, exact: bool = False):
+    """1/a (op 0), 1/sqrt(a) (1), sqrt(a) (2), and without the ends (0, infinity)
+    b/a (3), 1/a (4), 1/sqrt(a) (5), sqrt(a) (6) as the product build's kernels
+    form them; exact: CUDA's operators."""
+    a = np.ascontiguousarray(a, dtype=np.float64)
+    b = np.ascontiguousarray(np.ones_like(a) if b is None else b, dtype=np.float64)
+    out = np.empty_like(a)
+    rc = load(exact).echo_gpu_test_recip(op, len(a), _dp(a), _dp(b), _dp(out))
+    if rc:
+        raise RuntimeError(f"test_recip status {rc}")
+    return out
 
 
 def unit_offsets(nx: int, ny: int, nz: int, exact: bool = False) -> list[int]:

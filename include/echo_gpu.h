@@ -406,6 +406,11 @@ int echo_gpu_test_offsets(int nx, int ny, int nz, unsigned long long* off);
  * more than 2^29 cells or faces take, whatever its grid. */
 int echo_gpu_test_wide(EchoCtx* ctx);
 
+/* The product build's reciprocals on n operands: op 0 1/a, 1 1/sqrt(a), 2
+ * sqrt(a), and without the ends (0, infinity) 3 b/a, 4 1/a, 5 1/sqrt(a), 6
+ * sqrt(a); the parity build gives CUDA's own operators. */
+int echo_gpu_test_recip(int op, int n, const double* a, const double* b, double* out);
+
 /* Reconstruction of m pencils of length n (+ghosts) with REC_ALGO.
  * f is m rows of (n + 8) values, f[row*(n+8) + (i+4)] = f(i), i=-4..n+3;
  * gl/gr are m rows of n+1 faces (holib.f90:47-348). */
