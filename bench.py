@@ -641,23 +641,25 @@ def run_b200(args):
         torch.cuda.synchronize()
         e0 = torch.cuda.Event(enable_timing=True)
         e1 = torch.cuda.Event(enable_timing=True)
+        k0, _ = ev.run_counts()
         e0.record(stream)
         ev.run(args.steps)
         e1.record(stream)
         ev.sync()
         torch.cuda.synchronize()
         barrier()
+        k1, _ = ev.run_counts()
         ms = torch.tensor([e0.elapsed_time(e1)], dtype=torch.float64, device="cuda")
         if world > 1:
             dist.all_reduce(ms, op=dist.ReduceOp.MAX)
         st = ev.stats()
-        return ev, stream, float(ms.item()), st
+        return ev, stream, float(ms.item()), st, k1 - k0
 
     variants = {}
     names = {P.C2P_BRENT: "reference_brentm", P.C2P_NEWTON: "plain_newton", P.C2P_MLP: "mlp_seeded"}
     keep = None
     for algo in (P.C2P_BRENT, P.C2P_NEWTON, P.C2P_MLP):
-        ev, stream, ms, st = timed(algo)
+        ev, stream, ms, st, launches = timed(algo)
         it = st.c2p_iters / max(cfg0.ncell, 1)
         variants[names[algo]] = {
             "value": cfg0.ncell * args.steps * world / (ms / 1e3), "ms_per_step": ms / args.steps,
@@ -666,11 +668,11 @@ def run_b200(args):
             "seed_fallbacks_total": int(st.seed_fallbacks), "bracket_fallbacks_total": int(st.bracket_fallbacks),
             "errcode": int(st.errcode)}
         if algo == P.C2P_NEWTON:
-            keep = (ev, stream, ms, st)
+            keep = (ev, stream, ms, st, launches)
         else:
             ev.close()
     clocks = clk.stop()
-    ev, stream, ms_max, st = keep
+    ev, stream, ms_max, st, launches = keep
     value = variants["plain_newton"]["value"]
     prof = ev.profile_step()  # one real step, per-kernel device times
     ev.sync()
@@ -733,10 +735,6 @@ def run_b200(args):
         flop_step = sum(krec[k]["fp64_flop"] * n for k, (_, n) in prof.items() if k in krec and n)
     counters_src = {"file": os.path.relpath(COUNTERS, ROOT), "build_hash": cnt.get("build_hash"),
                     "this_build": CT.build_hash(), "same_build": fresh}
-    # one launch each per stage: the sweeps (with the stage's scalars), the update,
-    # the repair (which also ends the step)
-    launches_per_step = 3 * cfg0.nrk
-
     cpu = None
     if world == 1:
         rate, el, sample = cpu_rate(cfg0, tab, przero, threads=1, target_s=6.0, steps=2)
@@ -784,7 +782,7 @@ def run_b200(args):
         "batched": batched,
         "resistive": resistive,
         "ideal_hd": ideal_hd,
-        "gpu_launches": launches_per_step * args.steps,
+        "gpu_launches": launches,  # the timed region's, counted from its step graphs
         "clocks": clocks,
         "stats": {"errcode": st.errcode, "repairs": st.repairs, "t": st2.t, "dt": st.dt},
     }

@@ -44,6 +44,9 @@ struct EchoCtx {
   DevScalars* h_sc;         // pinned mirror
   cudaGraphExec_t graph[16];  // one per buffer-role key at step start
   bool graph_ok[16];
+  // kernel nodes of each graph and their thread blocks; what echo_gpu_run has
+  // launched of them (echo_gpu_run_counts)
+  long long graph_kernels[16], graph_blocks[16], run_kernels, run_blocks;
   // per-kernel timing (echo_gpu_profile_step): events recorded after each launch group
   std::vector<std::pair<int, cudaEvent_t>>* marks;
   EchoHyp* hyp;             // set up by echo_gpu_hyp_init

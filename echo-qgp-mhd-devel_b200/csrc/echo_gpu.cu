@@ -685,6 +685,32 @@ int echo_gpu_step(EchoCtx* c, double* dt, int* errcode) {
   return ECHO_OK;
 }
 
+// the kernel nodes of a graph and their thread blocks
+static int count_graph(cudaGraph_t gr, long long* kernels, long long* blocks) {
+  size_t n = 0;
+  CK(cudaGraphGetNodes(gr, nullptr, &n));
+  std::vector<cudaGraphNode_t> nodes(n);
+  CK(cudaGraphGetNodes(gr, nodes.data(), &n));
+  *kernels = *blocks = 0;
+  for (size_t i = 0; i < n; i++) {
+    cudaGraphNodeType type;
+    CK(cudaGraphNodeGetType(nodes[i], &type));
+    if (type != cudaGraphNodeTypeKernel) continue;
+    cudaKernelNodeParams k;
+    CK(cudaGraphKernelNodeGetParams(nodes[i], &k));
+    *kernels += 1;
+    *blocks += (long long)k.gridDim.x * k.gridDim.y * k.gridDim.z;
+  }
+  return ECHO_OK;
+}
+
+int echo_gpu_run_counts(EchoCtx* c, long long* kernels, long long* blocks) {
+  if (!c) return ECHO_ERR_ARG;
+  if (kernels) *kernels = c->run_kernels;
+  if (blocks) *blocks = c->run_blocks;
+  return ECHO_OK;
+}
+
 int echo_gpu_run(EchoCtx* c, int nsteps) {
   if (c && c->p.algo_solver == ECHO_C2P_MLP && !c->d_mlp_frag) return ECHO_ERR_ARG;  // no network loaded
   (void)cudaGetLastError();  // a failed launch of an earlier call must not be reported here
@@ -698,6 +724,8 @@ int echo_gpu_run(EchoCtx* c, int nsteps) {
       CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
       enqueue_step(c);  // records the launches and advances the roles
       CK(cudaStreamEndCapture(c->stream, &gr));
+      int r = count_graph(gr, &c->graph_kernels[key], &c->graph_blocks[key]);
+      if (r) return r;
       CK(cudaGraphInstantiate(&c->graph[key], gr, 0));
       cudaGraphDestroy(gr);
       c->graph_ok[key] = true;
@@ -705,6 +733,8 @@ int echo_gpu_run(EchoCtx* c, int nsteps) {
       advance_roles(c);
     }
     CK(cudaGraphLaunch(c->graph[key], c->stream));
+    c->run_kernels += c->graph_kernels[key];
+    c->run_blocks += c->graph_blocks[key];
   }
   CK(cudaGetLastError());
   return ECHO_OK;

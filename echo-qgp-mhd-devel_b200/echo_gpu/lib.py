@@ -101,6 +101,7 @@ FUNCTIONS = {
     "echo_gpu_test_c2p_seeded": (ctypes.c_int, [P, D, ctypes.c_int, ctypes.c_int, ctypes.c_double, ctypes.c_double,
                                                 F, F, D, D, I, I, I]),
     "echo_gpu_get_state": (ctypes.c_int, [P, P, P]),
+    "echo_gpu_run_counts": (ctypes.c_int, [P, LL, LL]),
     "echo_gpu_profile_step": (ctypes.c_int, [P, D, I]),
     "echo_gpu_set_stage": (ctypes.c_int, [P, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, I]),
     "echo_gpu_set_faces": (ctypes.c_int, [P, ctypes.c_int]),
@@ -278,6 +279,12 @@ class Evolve:
 
     def run(self, nsteps: int):
         self._check(self.lib.echo_gpu_run(self.h, nsteps), "run")
+
+    def run_counts(self) -> tuple[int, int]:
+        """Kernels, and their thread blocks, that run() has launched so far."""
+        k, b = ctypes.c_longlong(0), ctypes.c_longlong(0)
+        self._check(self.lib.echo_gpu_run_counts(self.h, ctypes.byref(k), ctypes.byref(b)), "run_counts")
+        return k.value, b.value
 
     def sync(self):
         self._check(self.lib.echo_gpu_sync(self.h), "sync")

@@ -337,6 +337,11 @@ int echo_gpu_hyp_init(EchoCtx* ctx, int freeze_type, double freeze_value);
 int echo_gpu_hyp_step(EchoCtx* ctx, int* n_elements, int* errcode);
 int echo_gpu_hyp_get(EchoCtx* ctx, double* out);
 
+/* No counterpart in the reference (measurement).  The kernels, and their thread
+ * blocks, that echo_gpu_run has launched on this context since its creation,
+ * counted from the kernel nodes of the step graphs it launched. */
+int echo_gpu_run_counts(EchoCtx* ctx, long long* kernels, long long* blocks);
+
 /* Runs one full step with a CUDA event after every launch group and returns
  * the device time per kernel class (ms[8]: faces x, faces y, faces z, stage
  * scalars, update+con2prim, repair(+smoothing), end of step, fused stage)
