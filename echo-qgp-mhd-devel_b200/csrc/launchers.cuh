@@ -12,15 +12,18 @@ namespace echo {
 // ---------------------------------------------------------------------------
 // kernel dispatch
 // ---------------------------------------------------------------------------
-// Tile of the sweeps (faces.cuh): 256 cells where that gives every SM two
-// blocks; 32 cells, with the block's further threads sharing the variables,
-// where it does not (201 x 201 viscous x / y sweep 28 / 25 us with 32 cells,
-// 25 / 23 with 256; 101 x 101 hydro 12 / 9 and 14 / 12).
-inline int sweep_lc(const EchoCtx* c, int mask) {
+// Tile of the sweeps (faces.cuh): 256 cells where those of a stage give each of
+// the 148 SMs two blocks; 32 cells, with the block's further threads sharing the
+// variables, where they do not (201 x 201 viscous x / y sweep 28 / 25 us with 32
+// cells, 25 / 23 with 256; 101 x 101 hydro 12 / 9 and 14 / 12).  By the grid
+// alone: sweeps launched one by one run the kernels, and give the bits, of those
+// in one launch.
+inline int sweep_lc(const EchoCtx* c) {
   if (c->wide) return 8;
+  const Grid& g = c->g;
   unsigned t = 0;
   for (int d = 0; d < 3; d++)
-    if (mask >> d & 1) t += tiles_of(c->g, d, 8, 4);
+    if ((d == 0 ? g.nx : d == 1 ? g.ny : g.nz) > 1) t += tiles_of(g, d, 8, 4);
   return t >= 2 * 148 ? 8 : 5;
 }
 
@@ -37,7 +40,7 @@ void launch_faces(EchoCtx* c, int mask, const ScalarArgs* last, bool check) {
   }
   // pencils of a tile of the y and eta sweeps: 16, or as many as leave
   // face_mode cells of each in a tile (echo_gpu_set_faces)
-  const int lc = sweep_lc(c, mask);
+  const int lc = sweep_lc(c);
   S.lw = c->face_mode == 8 ? lc - 3 : c->face_mode == 16 || lc == 8 ? lc - 4 : lc - 3;
   unsigned blocks = 0;
   for (int d = 0; d < 3; d++) {
