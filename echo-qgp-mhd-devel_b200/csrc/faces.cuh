@@ -6,7 +6,9 @@
 // shared memory.  Phase 2: the flux of a face takes the upper state of the cell
 // below and the lower state of the cell above.
 //
-// What bounds it: L1 and FP64 issue, in phases that the blocks of an SM overlap.
+// What bounds it: L1 and FP64 together (x / y / eta sweep of 97 x 97 x 81 ideal RMHD:
+// L1 70 / 61 / 55 % of its peak, FP64 pipe 44 / 47 / 44 %, issue 42 / 45 / 43 %), in
+// phases that the 21 to 23 warps of an SM overlap in part.
 // One thread per face with all its variables in registers (the arrangement
 // before) evaluated the smoothness indicators of a cell twice, unrolled every
 // variable into one body and spilled about 600 bytes a thread at the 72
@@ -28,6 +30,10 @@
 // them bounds it.
 #pragma once
 
+// Variables of phase 1 unrolled together.  Measured, 1 / 2 / 3, us for the passes
+// of whole steps: ideal RMHD 97 x 97 x 81 4796 / 4771 / 4761, resistive
+// 193 x 193 x 129 19453 / 19466 / 19517, hydro MPE5 75 x 67 x 49 1002 / 1012 / 1026,
+// viscous 61 x 57 x 41 877 / 887 / 900.
 #ifndef ECHO_SWEEP_UNROLL
 #define ECHO_SWEEP_UNROLL 2
 #endif
@@ -600,7 +606,11 @@ template <int KIND>
 __host__ __device__ constexpr int sweep_threads(int lc) {
   return 256 / sweep_cpt<KIND>(lc);
 }
-// blocks of an SM: the register bound that was fastest
+// Blocks of an SM, the register bound.  Measured with one fewer / this / one more,
+// us for the passes of whole steps: ideal RMHD 97 x 97 x 81 4824 / 4771 / 4929,
+// hydro MPE5 75 x 67 x 49 1067 / 1012 / 1020, viscous 61 x 57 x 41 980 / 887 / 934,
+// resistive 193 x 193 x 129 21279 / 19466 / 22144; small tiles (hydro 101 x 101)
+// 2359 / 2030 / 2055.
 #ifndef ECHO_SWEEP_MINB
 #define ECHO_SWEEP_MINB 6
 #endif
@@ -613,9 +623,12 @@ __host__ __device__ constexpr int sweep_threads(int lc) {
 #ifndef ECHO_SWEEP_MINB_RES
 #define ECHO_SWEEP_MINB_RES 4
 #endif
+#ifndef ECHO_SWEEP_MINB_SMALL
+#define ECHO_SWEEP_MINB_SMALL 3
+#endif
 template <int KIND>
 constexpr int sweep_minb(int lc) {
-  return lc != 8             ? 3
+  return lc != 8             ? ECHO_SWEEP_MINB_SMALL
          : KIND == KIND_HD   ? ECHO_SWEEP_MINB_HD
          : KIND == KIND_VISC ? ECHO_SWEEP_MINB_VISC
          : KIND == KIND_RES  ? ECHO_SWEEP_MINB_RES

@@ -712,7 +712,7 @@ __device__ __forceinline__ void mlp_seed(const MlpDev& net, const Metric& M, boo
 // runs, the spatial derivatives of u^mu in dv[NDER] (the rest zero); it
 // adds the lagged time derivatives, the sources, and does the RK
 // combination or writes du (MODE_RHS), then con2prim.  update_cell reads
-// the face fluxes of the three sweep kernels; the fused stage kernel
+// the face fluxes of the sweeps; the fused stage kernel
 // computes them itself (stage.cuh).
 template <int KIND, bool SEED, bool IMEX, int ALGO>
 __device__ __forceinline__ void update_finish(const UpdateArgs& A, size_t c, bool active, int ix, int iy, int iz,
